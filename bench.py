@@ -143,6 +143,9 @@ BYTES_PER_CELL = {
     "vel_phy_rtmfwd": 4 * (6 + 1 + 3) + 4 * 3,
     "vel_phy_fwd": 4 * (6 + 1 + 3) + 4 * 3,
     "stress_phy_bwd": 4 * (3 + 2 + 7) + 4 * 7,
+    "stress_tile_bwd": 4 * (3 + 2 + 7) + 4 * 7,
+    "vel_tile_bwd": 4 * (6 + 1 + 3) + 4 * 3,
+    "pvel_image": 4 * (2 + 1 + 6 + 6 + 5) + 4 * (6 + 5),
     "stress_phy_rev": 4 * (3 + 2 + 7) + 4 * 7,
     "stress_phy_rtmfwd": 4 * (3 + 2 + 7) + 4 * 7,
     "stress_phy_fwd": 4 * (3 + 2 + 6) + 4 * 6,
@@ -154,7 +157,8 @@ BYTES_PER_CELL = {
 # can move; the full-gridext kernels add CPML memory variables at the rim
 FOOTPRINT = {
     "vel_phy_bwd_image": (25, 11), "vel_phy_rev": (14, 6), "vel_phy_rtmfwd": (10, 3), "vel_phy_fwd": (10, 3),
-    "vel_fz_rtmfwd": (10, 3), "vel_fz_fwd": (10, 3),
+    "vel_fz_rtmfwd": (10, 3), "vel_fz_fwd": (10, 3), "vel_tile_rtmfwd": (10, 3), "vel_tile_fwd": (10, 3),
+    "vel_tile_rev": (10, 3), "vel_tile_bwd": (10, 3), "pvel_image": (20, 11), "stress_tile_bwd": (12, 7),
     "stress_phy_bwd": (12, 7), "stress_phy_rev": (12, 7), "stress_phy_rtmfwd": (12, 7),
     "stress_fz_rev": (12, 7), "stress_fz_rtmfwd": (12, 7),
 }
@@ -209,7 +213,10 @@ FUSED = {"stress_fz_fwd": ("stress_phy_fwd", "stress_pml"),
          "stress_fz_rtmfwd": ("stress_phy_rtmfwd", "stress_pml_sau"),
          "stress_fz_rev": ("stress_phy_rev", "stress_pml_sau"),
          "vel_fz_fwd": ("vel_phy_fwd", "vel_pml"),
-         "vel_fz_rtmfwd": ("vel_phy_rtmfwd", "vel_pml")}
+         "vel_fz_rtmfwd": ("vel_phy_rtmfwd", "vel_pml"),
+         "vel_tile_fwd": ("vel_phy_fwd", "vel_pml"),
+         "vel_tile_rtmfwd": ("vel_phy_rtmfwd", "vel_pml"),
+         "vel_tile_rev": ("vel_phy_fwd", "vel_pml")}
 
 
 def kernel_bytes(s, name):

@@ -139,7 +139,19 @@ GridDev make_layout(const jv_grid &grid, size_t *field_elems) {
     g.m = m;
     g.px = grid.nx; g.py = grid.ny; g.pz = grid.nz;
     g.nx = grid.nx + 2 * m; g.ny = grid.ny + 2 * m; g.nz = grid.nz + 2 * m;
+    // The first column's offset in its row: the first gridphy column on a
+    // 128-byte line, unless another offset (16-byte groups stay aligned)
+    // lets the tile kernels' 32-column tiles, which start on such lines,
+    // cover the rows with fewer tiles: four updates a migration step run over
+    // gridext, three over gridphy.
+    auto tiles = [&](int xo) {
+        const int f = (xo + 2) / 32 * 32, p = (xo + m) / 32 * 32;
+        return 4 * ((xo + g.nx - 2 - f + 31) / 32) + 3 * ((xo + m + g.px - p + 31) / 32);
+    };
     g.xoff = (32 - (m % 32)) % 32;
+    const int first = g.xoff;
+    for (int xo = first % 4; xo < 32; xo += 4)
+        if (tiles(xo) < tiles(g.xoff)) g.xoff = xo;
     g.sy = round_up(g.xoff + g.nx, 32);
     g.sz = g.sy * g.ny;
     g.dx = grid.dx; g.dy = grid.dy; g.dz = grid.dz;
@@ -219,13 +231,17 @@ void pml_axis_tables(const GridDev &g, float fm, std::vector<float4> t[3]) {
     }
 }
 
-int upload_all_coefficients() {
-    float list[5][4] = {};
-    for (int o = 1; o <= 4; o++) {
-        double c[4];
-        diff_coeff(o, c);
-        for (int i = 0; i < o; i++) list[o][i] = (float)c[i];
+void staggered_taps(float list[5][4]) {
+    for (int o = 0; o <= 4; o++) {
+        double c[4] = {};
+        if (o) diff_coeff(o, c);
+        for (int i = 0; i < 4; i++) list[o][i] = i < o ? (float)c[i] : 0.f;
     }
+}
+
+int upload_all_coefficients() {
+    float list[5][4];
+    staggered_taps(list);
     double c2[2];
     diff_coeff(2, c2);
     const float dc2[2] = {(float)c2[0], (float)c2[1]};
@@ -282,13 +298,13 @@ std::vector<SegDev> vowr_segments(const GridDev &g, int r, long long *per_step, 
 size_t footprint_bytes(const jv_grid &grid, int nt, int rec_width, bool rtm, int precision) {
     size_t fe = 0;
     const GridDev g = make_layout(grid, &fe);
-    long long psi = 0;
-    make_pml_slabs(g, 1, &psi);
     const size_t nphy = (size_t)grid.nx * grid.ny * grid.nz;
     size_t b = (4 * fe + 32) * sizeof(float);                 // model
     b += (kNumFld * fe + 32) * sizeof(float);                 // forward wavefield
-    b += (size_t)psi * sizeof(float);                         // its memory variables
-    b += (size_t)2 * fz_psi_floats(g) * sizeof(float);        // the full-gridext kernels' ones
+    long long slabs = 0;
+    make_pml_slabs(g, 1, &slabs);
+    const size_t psi = (size_t)(tiles_fit(g) ? tile_psi_floats(g) : slabs) * sizeof(float);
+    b += psi;                                                 // its memory variables
     b += 5 * nphy * sizeof(double);                           // stacks
     b += 16 * ((size_t)grid.nx + grid.ny + grid.nz + 2 * grid.pml * 3) + (1 << 20);  // tables, state, slack
     if (rtm) {
@@ -296,7 +312,7 @@ size_t footprint_bytes(const jv_grid &grid, int nt, int rec_width, bool rtm, int
         const bool s16 = precision == JV_BF16 || precision == JV_FP16;
         const std::vector<SegDev> segs = vowr_segments(g, rec_width, &per, &blk, !s16);
         const size_t nslot = nt > 1 ? nt - 1 : 0;
-        b += (kNumFld * fe + 32) * sizeof(float) + (size_t)(psi + 2 * fz_psi_floats(g)) * sizeof(float);  // receiver wavefield
+        b += (kNumFld * fe + 32) * sizeof(float) + psi;                             // receiver wavefield
         b += (size_t)per * nslot * (s16 ? sizeof(uint16_t) : sizeof(float));      // boundary store
         if (s16) b += (nslot + 2) * segs.size() * sizeof(float);                    // its per-box scales
         b += 5 * ((nphy + 63) / 64 * 64) * sizeof(float);                           // shot image
@@ -393,7 +409,8 @@ Status Engine::autotune(bool neutral) {
     cudaDeviceProp prop{};
     JV_CU(cudaGetDeviceProperties(&prop, dev));
     const std::array<long long, 7> key = {grid_.nx, grid_.ny, grid_.nz, grid_.pml, prop.multiProcessorCount,
-                                          (long long)prop.totalGlobalMem, neutral ? 1 : 0};
+                                          (long long)prop.totalGlobalMem,
+                                          neutral ? 10 + kc_.variant : 0};
     Status st{};
     auto apply = [&](const Cand &c) {
         kc_.variant = c.variant;
@@ -402,13 +419,11 @@ Status Engine::autotune(bool neutral) {
             kc_.gx = c.gx;
             kc_.gy = 0;
         }
-        if (c.variant == 4 && fullF_.ok && c.q > 0 && c.q != fullF_.geo.Q) {
+        if (c.variant == 4 && tileF_.ok && c.q > 0 && c.q != tileF_.geo.Q) {
             kc_.fzq = c.q;
-            const int e = k_make_full_maps(g_, F_, lam_, mu_, vp_, bdt_, axis_d_, fzpsiF_, zm_err_, kc_.fzq, &fullF_);
-            if (e != 0 || !fullF_.ok) st = bad(JV_ECUDA, "variant-4 descriptors for the measured choice");
+            st = make_tiles();
         }
-        use_full_ = c.variant == 4 && fullF_.ok;
-        vel_full_ = use_full_ && fullF_.geo.NTX == 1;
+        tiles_ = c.variant == 4 && tileF_.ok;
     };
     {
         std::lock_guard<std::mutex> l(mu);
@@ -419,12 +434,12 @@ Status Engine::autotune(bool neutral) {
         }
     }
     std::vector<Cand> cands;
-    if (fullF_.ok) {
+    if (tileF_.ok) {
         if (kc_.fzq > 0) {
-            cands.push_back({4, 4, fullF_.geo.Q});
+            cands.push_back({4, 4, tileF_.geo.Q});
         } else {
             for (int k = 0; k < 3; k++)
-                if (fullF_.qcand[k] > 0) cands.push_back({4, 4, fullF_.qcand[k]});
+                if (tileF_.qcand[k] > 0) cands.push_back({4, 4, tileF_.qcand[k]});
         }
     }
     if (neutral) {
@@ -450,7 +465,7 @@ Status Engine::autotune(bool neutral) {
         apply(c);
         JV_TRY(st);
         JV_TRY(zero_wave(F_, 9));
-        JV_TRY(zero_psi(cpF_));
+        JV_TRY(zero_psi(false));
         JV_TRY(set_state(0, src, nullptr, nullptr));
         for (int i = 0; i < warm; i++) JV_TRY(launch_step(kStepModel, 0, true));
         JV_CU(cudaEventRecord(ev0_, stream_));
@@ -467,7 +482,7 @@ Status Engine::autotune(bool neutral) {
     }
     apply(pick);
     JV_TRY(st);
-    if (shape_free) {
+    if (shape_free && !tiles_) {
         const int ngx = (g_.px + 3) / 4, nb0 = (ngx + 63) / 64;
         float sbest = -1.f;
         for (int nb = std::max(1, nb0 - 1); nb <= nb0 + 1; nb++) {
@@ -496,7 +511,7 @@ Status Engine::autotune(bool neutral) {
         apply(pick);
     }
     JV_TRY(zero_wave(F_, kNumFld));
-    JV_TRY(zero_psi(cpF_));
+    JV_TRY(zero_psi(false));
     JV_CU(cudaStreamSynchronize(stream_));
     std::lock_guard<std::mutex> l(mu);
     cache[key] = pick;
@@ -548,18 +563,20 @@ Status Engine::alloc_all(const float *vp, const float *vs, const float *rho) {
             axis_d_[a] = (float4 *)p;
             JV_CU(cudaMemcpy(axis_d_[a], t[a].data(), t[a].size() * sizeof(float4), cudaMemcpyHostToDevice));
         }
+    }
+    if (kc_.variant == 4 && tiles_fit(g_)) {
+        tpsi_total_ = tile_psi_floats(g_);
+        JV_TRY(alloc(&p, (size_t)tpsi_total_ * sizeof(float)));
+        tpsiF_ = (float *)p;
+        JV_TRY(make_tiles());
+        tiles_ = tileF_.ok;
+        wide_ = g_.nx - 4 + 10 > 256;
+    }
+    // the slab layout's memory variables: the other variants, tried by the
+    // measured choice
+    if (!tiles_ || opt_.kernel_variant < 0) {
         JV_TRY(alloc(&p, (size_t)psi_total_ * sizeof(float)));
         cpF_ = make_cpml((float *)p);
-    }
-    if (kc_.variant == 4) {
-        fz_psi_total_ = 2 * fz_psi_floats(g_);  // velocity and stress sets
-        JV_TRY(alloc(&p, (size_t)fz_psi_total_ * sizeof(float)));
-        fzpsiF_ = (float *)p;
-        JV_K(k_make_full_maps(g_, F_, lam_, mu_, vp_, bdt_, axis_d_, fzpsiF_, zm_err_, kc_.fzq, &fullF_));
-        // the fused velocity update runs on one-tile grids, where it measured
-        // faster than the split kernels; x-tiled grids keep the split ones
-        use_full_ = fullF_.ok;
-        vel_full_ = fullF_.ok && fullF_.geo.NTX == 1;
     }
 
     // wavelet and step state
@@ -599,6 +616,17 @@ Status Engine::alloc_all(const float *vp, const float *vs, const float *rho) {
         }
     }
     JV_CU(cudaStreamSynchronize(stream_));
+    return Status{};
+}
+
+// the tile kernels' descriptors of every wavefield allocated so far
+Status Engine::make_tiles() {
+    JV_K(k_make_tile_maps(g_, F_, false, axis_d_, tpsiF_, zm_err_, kc_.fzq, &tileF_));
+    JV_K(k_make_tile_maps(g_, F_, true, axis_d_, nullptr, zm_err_, 0, &tileFB_));
+    if (R_.f[0]) {
+        JV_K(k_make_tile_maps(g_, R_, false, axis_d_, tpsiR_, zm_err_, kc_.fzq, &tileR_));
+        JV_K(k_make_tile_maps(g_, R_, true, axis_d_, nullptr, zm_err_, 0, &tileRB_));
+    }
     return Status{};
 }
 
@@ -709,11 +737,12 @@ CpmlDev Engine::make_cpml(float *psi) const {
     return c;
 }
 
-Status Engine::zero_psi(const CpmlDev &c) {
-    if (psi_total_ > 0) JV_CU(cudaMemsetAsync(c.psi, 0, (size_t)psi_total_ * sizeof(float), stream_));
-    // the axis-major stress memory variables of the full-gridext kernel
-    float *fz = c.psi == cpF_.psi ? fzpsiF_ : c.psi == cpR_.psi ? fzpsiR_ : nullptr;
-    if (fz) JV_CU(cudaMemsetAsync(fz, 0, (size_t)fz_psi_total_ * sizeof(float), stream_));
+Status Engine::zero_psi(bool receiver) {
+    const CpmlDev &c = receiver ? cpR_ : cpF_;
+    float *tp = receiver ? tpsiR_ : tpsiF_;
+    if (!tiles_ && c.psi && psi_total_ > 0)
+        JV_CU(cudaMemsetAsync(c.psi, 0, (size_t)psi_total_ * sizeof(float), stream_));
+    if (tiles_) JV_CU(cudaMemsetAsync(tp, 0, (size_t)tpsi_total_ * sizeof(float), stream_));
     return Status{};
 }
 
@@ -831,15 +860,14 @@ Status Engine::launch_step(int kind, int off, bool advance) {
     const int rw = opt_.rec_width;
     switch (kind) {
     case kStepModel:
-        if (vel_full_) {
-            JV_L("vel_fz_fwd", k_vel_full(g_, F_, dt, fullF_, s));
+        if (tiles_) {
+            if (wide_) folded("vel_pml"), folded("vel_phy_fwd");
+            JV_L(wide_ ? "vel_tile_fwd" : "vel_fz_fwd", k_vel_tile(kFwd, g_, F_, bdt_, vp_, dt, rw, tileF_, s));
+            JV_L("stress_fz_fwd",
+                 k_stress_tile(kFwd, g_, F_, lam_, mu_, vp_, dt, rw, wavelet_, st_, off, tileF_, s));
         } else {
             JV_L("vel_pml", k_vel_pml(g_, cpF_, F_, bdt_, vp_, kc_, s));
             JV_L("vel_phy_fwd", k_vel_phy(kFwd, g_, F_, bdt_, dt, rw, nullptr, nullptr, kc_, s));
-        }
-        if (use_full_) {
-            JV_L("stress_fz_fwd", k_stress_full(kFwd, g_, F_, dt, wavelet_, st_, off, fullF_, s));
-        } else {
             JV_L("stress_pml", k_stress_pml(g_, cpF_, F_, lam_, mu_, vp_, 0, kc_, s));
             JV_L("stress_phy_fwd",
                  k_stress_phy(kFwd, g_, F_, lam_, mu_, dt, rw, wavelet_, st_, off, kc_, s, &mapsF_));
@@ -848,17 +876,16 @@ Status Engine::launch_step(int kind, int off, bool advance) {
         if (advance) JV_L("step_advance", k_step_advance(st_, +1, s));
         break;
     case kStepRtmFwd:
-        if (vel_full_) {
-            JV_L("vel_fz_rtmfwd", k_vel_full(g_, F_, dt, fullF_, s));
+        if (tiles_) {
+            if (wide_) folded("vel_pml"), folded("vel_phy_rtmfwd");
+            JV_L(wide_ ? "vel_tile_rtmfwd" : "vel_fz_rtmfwd", k_vel_tile(kRtmFwd, g_, F_, bdt_, vp_, dt, rw, tileF_, s));
+            // the boundary boxes lie in the absorbing layers: pack them after their update
+            JV_L("stress_fz_rtmfwd",
+                 k_stress_tile(kRtmFwd, g_, F_, lam_, mu_, vp_, dt, rw, wavelet_, st_, off, tileF_, s));
+            JV_L("vowr_pack", k_vowr(g_, F_, vowr_, st_, off, 1, 0, s));
         } else {
             JV_L("vel_pml", k_vel_pml(g_, cpF_, F_, bdt_, vp_, kc_, s));
             JV_L("vel_phy_rtmfwd", k_vel_phy(kRtmFwd, g_, F_, bdt_, dt, rw, nullptr, nullptr, kc_, s));
-        }
-        if (use_full_) {
-            // the boundary boxes lie in the absorbing layers: pack them after their update
-            JV_L("stress_fz_rtmfwd", k_stress_full(kRtmFwd, g_, F_, dt, wavelet_, st_, off, fullF_, s));
-            JV_L("vowr_pack", k_vowr(g_, F_, vowr_, st_, off, 1, 0, s));
-        } else {
             JV_L("stress_pml_sau", k_stress_pml(g_, cpF_, F_, lam_, mu_, vp_, 1, kc_, s));
             JV_L("vowr_pack", k_vowr(g_, F_, vowr_, st_, off, 1, 0, s));
             JV_L("stress_phy_rtmfwd",
@@ -870,19 +897,28 @@ Status Engine::launch_step(int kind, int off, bool advance) {
         // UPDATE 1: source subtraction (fused) + backward stress, receiver
         // injection + reverse velocity, stress boundary layers of step it-1
         JV_L("inject_rec", k_inject_rec(R_, rec_d_, nrec_, nt_, st_, off, s));
-        JV_L("stress_phy_bwd", k_stress_phy(kBwd, g_, F_, lam_, mu_, -dt, rw, wavelet_, st_, off, kc_, s, &mapsF_));
-        // the receiver side's velocity update: absorbing layers, then gridphy
-        // (with its P-wave velocities, the full-gridext form measured no
-        // faster on cfg2 and slower on x-tiled grids)
-        JV_L("vel_pml", k_vel_pml(g_, cpR_, R_, bdt_, vp_, kc_, s));
-        JV_L("vel_phy_rev", k_vel_phy(kRev, g_, R_, bdt_, dt, rw, nullptr, nullptr, kc_, s));
+        if (tiles_) {
+            JV_L("stress_tile_bwd",
+                 k_stress_tile(kBwd, g_, F_, lam_, mu_, vp_, -dt, rw, wavelet_, st_, off, tileFB_, s));
+            // the receiver side's velocities, absorbing layers included; its
+            // P-wave velocities follow in the imaging kernel
+            folded("vel_pml"), folded("vel_phy_rev");
+            JV_L("vel_tile_rev", k_vel_tile(kRev, g_, R_, bdt_, vp_, dt, rw, tileR_, s));
+        } else {
+            JV_L("stress_phy_bwd",
+                 k_stress_phy(kBwd, g_, F_, lam_, mu_, -dt, rw, wavelet_, st_, off, kc_, s, &mapsF_));
+            JV_L("vel_pml", k_vel_pml(g_, cpR_, R_, bdt_, vp_, kc_, s));
+            JV_L("vel_phy_rev", k_vel_phy(kRev, g_, R_, bdt_, dt, rw, nullptr, nullptr, kc_, s));
+        }
         JV_L("vowr_unpack", k_vowr(g_, F_, vowr_, st_, off - 1, 0, 2, s));
         // UPDATE 2: backward velocity with the imaging condition fused,
         // reverse stress, velocity boundary layers of step it-1
-        JV_L("vel_phy_bwd_image", k_vel_phy(kBwd, g_, F_, bdt_, -dt, rw, &R_, &shot_img_, kc_, s));
-        if (fullR_.ok) {
-            JV_L("stress_fz_rev", k_stress_full(kRev, g_, R_, dt, wavelet_, st_, off, fullR_, s));
+        if (tiles_) {
+            JV_L("vel_tile_bwd", k_vel_tile(kBwd, g_, F_, bdt_, vp_, dt, rw, tileFB_, s));
+            JV_L("pvel_image", k_pvel_tile(g_, &F_, &tileFB_, R_, tileRB_, true, bdt_, rw, &shot_img_, s));
+            JV_L("stress_fz_rev", k_stress_tile(kRev, g_, R_, lam_, mu_, vp_, dt, rw, wavelet_, st_, off, tileR_, s));
         } else {
+            JV_L("vel_phy_bwd_image", k_vel_phy(kBwd, g_, F_, bdt_, -dt, rw, &R_, &shot_img_, kc_, s));
             JV_L("stress_pml_sau", k_stress_pml(g_, cpR_, R_, lam_, mu_, vp_, 1, kc_, s));
             JV_L("stress_phy_rev",
                  k_stress_phy(kRev, g_, R_, lam_, mu_, dt, rw, wavelet_, st_, off, kc_, s, &mapsR_));
@@ -959,7 +995,7 @@ Status Engine::forward(int shot, float *d_vx, float *d_vy, float *d_vz) {
     float *tr[3] = {d_vx, d_vy, d_vz};
     JV_CU(cudaEventRecord(ev0_, stream_));
     JV_TRY(zero_wave(F_, 9));
-    JV_TRY(zero_psi(cpF_));
+    JV_TRY(zero_psi(false));
     JV_TRY(set_state(0, src, tr, nullptr));
     JV_TRY(run_loop(kStepModel, nt_));
     JV_CU(cudaEventRecord(ev1_, stream_));
@@ -983,12 +1019,13 @@ Status Engine::rtm_prepare() {
         JV_CU(cudaMemsetAsync(p, 0, kGuard * sizeof(float), stream_));
         for (int f = 0; f < kNumFld; f++) R_.f[f] = (float *)p + kGuard + f * field_elems_;
         if (kc_.variant >= 3) JV_K(k_make_wave_maps(g_, R_, lam_, mu_, zm_err_, &mapsR_));
-        JV_TRY(alloc(&p, (size_t)psi_total_ * sizeof(float)));
-        cpR_ = make_cpml((float *)p);
-        if (kc_.variant == 4) {
-            JV_TRY(alloc(&p, (size_t)fz_psi_total_ * sizeof(float)));
-            fzpsiR_ = (float *)p;
-            JV_K(k_make_full_maps(g_, R_, lam_, mu_, vp_, bdt_, axis_d_, fzpsiR_, zm_err_, kc_.fzq, &fullR_));
+        if (tiles_) {
+            JV_TRY(alloc(&p, (size_t)tpsi_total_ * sizeof(float)));
+            tpsiR_ = (float *)p;
+            JV_TRY(make_tiles());
+        } else {
+            JV_TRY(alloc(&p, (size_t)psi_total_ * sizeof(float)));
+            cpR_ = make_cpml((float *)p);
         }
     }
     if (!shot_img_.ip) {
@@ -1062,7 +1099,7 @@ Status Engine::rtm_forward_pass(int shot) {
     JV_TRY(rtm_prepare());
     // forward with boundary store (rtm_forward)
     JV_TRY(zero_wave(F_, kNumFld));
-    JV_TRY(zero_psi(cpF_));
+    JV_TRY(zero_psi(false));
     JV_TRY(set_state(0, src, nullptr, nullptr));
     JV_TRY(run_loop(kStepRtmFwd, nt_));
     // reconstruction check: the source wavefield's FP64 energy over gridphy
@@ -1083,7 +1120,7 @@ Status Engine::rtm_reverse_begin(int shot, const float *d_ox, const float *d_oy,
     const float *obs[3] = {d_ox, d_oy, d_oz};
     // time reverse: backward (reconstruction) + reverse (receivers) + image
     JV_TRY(zero_wave(R_, kNumFld));
-    JV_TRY(zero_psi(cpR_));
+    JV_TRY(zero_psi(true));
     JV_TRY(set_state(nt_ - 1, src, nullptr, obs));
     JV_CU(cudaMemsetAsync(shot_img_.ip, 0, 5 * shot_img_pitch_ * sizeof(float), stream_));
     rev_open_ = true;
@@ -1104,18 +1141,36 @@ Status Engine::rtm_reverse_op(int op, int it) {
     switch (op) {
     case JV_OP_INJECT_RECEIVERS: JV_K(k_inject_rec(R_, rec_d_, nrec_, nt_, st_, 0, s)); break;
     case JV_OP_BACKWARD_STRESS:
-        JV_K(k_stress_phy(kBwd, g_, F_, lam_, mu_, -dt, rw, wavelet_, st_, 0, kc_, s, &mapsF_));
+        if (tiles_) JV_K(k_stress_tile(kBwd, g_, F_, lam_, mu_, vp_, -dt, rw, wavelet_, st_, 0, tileFB_, s));
+        else JV_K(k_stress_phy(kBwd, g_, F_, lam_, mu_, -dt, rw, wavelet_, st_, 0, kc_, s, &mapsF_));
         break;
-    case JV_OP_REVERSE_VEL_PML: JV_K(k_vel_pml(g_, cpR_, R_, bdt_, vp_, kc_, s)); break;
-    case JV_OP_REVERSE_VEL: JV_K(k_vel_phy(kRev, g_, R_, bdt_, dt, rw, nullptr, nullptr, kc_, s)); break;
+    case JV_OP_REVERSE_VEL_PML:
+        // folded into the tile kernel of JV_OP_REVERSE_VEL where that one runs
+        if (!tiles_) JV_K(k_vel_pml(g_, cpR_, R_, bdt_, vp_, kc_, s));
+        break;
+    case JV_OP_REVERSE_VEL:
+        if (tiles_) {
+            JV_K(k_vel_tile(kRev, g_, R_, bdt_, vp_, dt, rw, tileR_, s));
+            JV_K(k_pvel_tile(g_, nullptr, nullptr, R_, tileRB_, true, bdt_, rw, nullptr, s));
+        } else {
+            JV_K(k_vel_phy(kRev, g_, R_, bdt_, dt, rw, nullptr, nullptr, kc_, s));
+        }
+        break;
     case JV_OP_INJECT_BOUNDARY_STRESS: JV_K(k_vowr(g_, F_, vowr_, st_, 0, 0, 2, s)); break;
-    case JV_OP_BACKWARD_VEL_IMAGE: JV_K(k_vel_phy(kBwd, g_, F_, bdt_, -dt, rw, &R_, &shot_img_, kc_, s)); break;
+    case JV_OP_BACKWARD_VEL_IMAGE:
+        if (tiles_) {
+            JV_K(k_vel_tile(kBwd, g_, F_, bdt_, vp_, dt, rw, tileFB_, s));
+            JV_K(k_pvel_tile(g_, &F_, &tileFB_, R_, tileRB_, false, bdt_, rw, &shot_img_, s));
+        } else {
+            JV_K(k_vel_phy(kBwd, g_, F_, bdt_, -dt, rw, &R_, &shot_img_, kc_, s));
+        }
+        break;
     case JV_OP_REVERSE_STRESS_PML:
-        // folded into the full-gridext stress kernel where that one runs
-        if (!fullR_.ok) JV_K(k_stress_pml(g_, cpR_, R_, lam_, mu_, vp_, 1, kc_, s));
+        // folded into the tile kernel of JV_OP_REVERSE_STRESS where that one runs
+        if (!tiles_) JV_K(k_stress_pml(g_, cpR_, R_, lam_, mu_, vp_, 1, kc_, s));
         break;
     case JV_OP_REVERSE_STRESS:
-        if (fullR_.ok) JV_K(k_stress_full(kRev, g_, R_, dt, wavelet_, st_, 0, fullR_, s));
+        if (tiles_) JV_K(k_stress_tile(kRev, g_, R_, lam_, mu_, vp_, dt, rw, wavelet_, st_, 0, tileR_, s));
         else JV_K(k_stress_phy(kRev, g_, R_, lam_, mu_, dt, rw, wavelet_, st_, 0, kc_, s, &mapsR_));
         break;
     case JV_OP_INJECT_BOUNDARY_VEL: JV_K(k_vowr(g_, F_, vowr_, st_, 0, 0, 1, s)); break;

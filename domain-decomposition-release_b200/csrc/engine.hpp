@@ -14,6 +14,7 @@
 
 #include "jv/jv.h"
 #include "jv_internal.hpp"
+#include "tile.hpp"
 
 namespace jv {
 
@@ -37,7 +38,7 @@ void set_last_error(const std::string &m);
 jv_status rtm_self_modelled(jv_ctx *c, int shot);
 
 // Pitched gridext layout of a gridphy + pml problem (elem = base + xoff +
-// i + sy*j + sz*k, first gridphy column 128-byte aligned); *field_elems =
+// i + sy*j + sz*k, first gridphy column 16-byte aligned); *field_elems =
 // floats of one field array (gridext plus tail slack for the aligned
 // x groups of the absorbing-layer kernels).
 GridDev make_layout(const jv_grid &grid, size_t *field_elems);
@@ -123,6 +124,7 @@ class Engine {
     Status run_loop(int kind, int nsteps);
     Status launch_step(int kind, int off, bool advance);
     Status autotune(bool neutral);
+    Status make_tiles();
 
   public:
     // the options this context runs with, the kernel choice as made
@@ -133,7 +135,7 @@ class Engine {
         o->pml_min_blocks = kc_.pml_minb;
         o->planes_per_thread = kc_.zp;
         o->pml_planes_per_thread = kc_.pml_zp;
-        o->run_chunks = use_full_ ? fullF_.geo.Q : 0;
+        o->run_chunks = tiles_ ? tileF_.geo.Q : 0;
         o->tile_gx = kc_.gx;
         o->tile_gy = kc_.gy;
     }
@@ -141,7 +143,7 @@ class Engine {
   private:
     Status cu(cudaError_t e, const char *what) const;
     Status zero_wave(const WaveDev &w, int nfld);
-    Status zero_psi(const CpmlDev &c);
+    Status zero_psi(bool receiver);
     Status set_state(int it, long long src, float *const tr[3], const float *const obs[3]);
     Status rtm_prepare();
     Status reverse_end_launch();
@@ -161,9 +163,11 @@ class Engine {
     GridDev g_{};
     KCfg kc_{};
     WaveMaps mapsF_{}, mapsR_{};  // TMA descriptors of the velocity fields (variant 3)
-    FullMaps fullF_{}, fullR_{};  // TMA descriptors of the full-gridext stress kernel (variant 4)
-    float *fzpsiF_ = nullptr, *fzpsiR_ = nullptr;  // its axis-major stress memory variables
-    long long fz_psi_total_ = 0;                   // floats of one of them
+    // variant 4's tile kernels: the wavefields over gridext, and over gridphy
+    // (the source reconstruction, and the P-wave velocities of both)
+    TileMaps tileF_{}, tileR_{}, tileFB_{}, tileRB_{};
+    float *tpsiF_ = nullptr, *tpsiR_ = nullptr;  // their axis-major memory variables
+    long long tpsi_total_ = 0;                   // floats of one of them
     double *energy_d_ = nullptr;          // device: the two energies of the reconstruction check
     double recon_energy_[2] = {0.0, 0.0};  // host copy after each RTM shot
 
@@ -176,8 +180,8 @@ class Engine {
     }
 
   private:
-    bool use_full_ = false;                        // the stress update of absorbing steps runs in stress_fz
-    bool vel_full_ = false;                        // the forward passes' velocity update runs in vel_fz
+    bool tiles_ = false;          // the time loops run variant 4's tile kernels
+    bool wide_ = false;           // a gridext row is wider than one 256-float box
     int *zm_err_ = nullptr;       // device flag of variant 3's bounded waits
     Status check_zm_err();
     size_t field_elems_ = 0;  // elements per pitched field
@@ -230,6 +234,10 @@ class Engine {
     std::vector<cudaEvent_t> prof_pool_;
     size_t prof_used_ = 0;
     int prof_id(const char *name);
+    // a phase that another phase's kernel carries: listed with no launches
+    void folded(const char *name) {
+        if (prof_) prof_id(name);
+    }
     cudaEvent_t prof_event();
     Status prof_collect();
 

@@ -4,8 +4,10 @@
 //   Every wavefield component and model parameter covers gridext
 //   (gridphy + pml cells per face) in one pitched array:
 //       elem(i, j, k) = base + xoff + i + sy * j + sz * k
-//   with the row pitch sy a multiple of 32 floats and xoff chosen so that
-//   the first gridphy column (i = pml) starts on a 128-byte boundary.
+//   with the row pitch sy a multiple of 32 floats and xoff chosen (make_layout)
+//   so that the first gridphy column (i = pml) starts on a 16-byte boundary,
+//   on a 128-byte one unless the tile kernels cover the rows with fewer
+//   tiles otherwise.
 //   Absorbing-layer memory variables live only in the six boundary slabs
 //   (slab-local dense indexing), not on the full grid.
 #pragma once
@@ -147,59 +149,6 @@ struct WaveMaps {
     int *err = nullptr;  // device flag: a bounded wait in the kernel ran out
 };
 
-// Geometry of the full-gridext stress kernel (variant 4).
-//  - x tiles: tile xt holds the physical x pairs [xt TPP, (xt+1) TPP) of the
-//    hxi = px/2, the first also the low absorbing strip [2, m), the last the
-//    high one [m+px, nx-2) (one tile: both); hxe: absorbing pairs a tile
-//    row carries (m-2 with one tile, else (m-2)/2); tpad: 4 TPP rounded up
-//    to whole warps (4 TPP where the rounding alone would take the tile
-//    past one CTA), the first thread of the absorbing pairs; corew: the
-//    core box width (the widest tile's).  ytiles, nzi: 4-row tiles over y in
-//    [2, ny-2), planes z in [2, nz-2).
-//  - The stress memory variables of this kernel are axis-major: per axis
-//    three arrays over the cells that absorb on that axis, rows packed
-//    (x arrays [t][z-2][y-2][xc], pitch PX over xc = the W absorbing x
-//    columns; y arrays [t][z-2][yc][x-2] and z arrays [t][zc][y-2][x-2],
-//    pitch PY over x-2), so that a tile's memory variables arrive by TMA
-//    with its fields (y and z boxes PB wide, from the tile's first cell
-//    rounded down to 16 bytes).  W = 2 (m - 2) absorbing indices per axis.
-//  - Runs: each tile's planes are cut into Q chunks of L planes (the last
-//    one padded with idle items); run r = chunk * (NTX ytiles) + tile, tile
-//    = yt NTX + xt, and CTA b takes runs b, b + grid, ...  Neighbouring CTAs
-//    then march neighbouring tiles through the same planes together, so
-//    halo rows are shared in L2.
-struct FzGeo {
-    int corew;
-    int hxi, hxe, tpad;
-    int NTX, TPP;       // x tiles; physical x pairs per tile
-    int ytiles, nzi;
-    int PX, PY, PB, W;  // PB: width of a y/z memory-variable box
-    int Q, L, R;
-    float *psx, *psy, *psz;
-    const float4 *ax[3];
-};
-
-// floats of one set (3 axes x 3 arrays) of axis-major memory variables; a
-// wavefield holds two, the velocity set first, then the stress set
-long long fz_psi_floats(const GridDev &g);
-
-// TMA descriptors of the full-gridext stress kernel of one wavefield
-struct FullMaps {
-    FieldMap halo[3];             // vx vy vz
-    FieldMap core[kZmCore + 1];   // vx vy vz, lam, mu, vp, sxx syy szz sxy sxz syz, sau
-    FieldMap psi[3];              // the x, y and z memory-variable arrays (4-D: 3 arrays each)
-    // the velocity kernel's: halo planes sxy syy syz, bands sxx sxz, core
-    // tiles rho vp vx vy vz, window feed sxz syz szz, memory variables
-    FieldMap vhalo[3], vband[2], vcore[5], vfeed[3], vpsi[3];
-    bool ok = false;              // false: variant 4 is not available for this grid
-    FzGeo geo{}, vgeo{};          // stress and velocity kernels (their memory-variable sets differ)
-    int threads = 0;
-    int grid = 0;
-    size_t smem = 0, vsmem = 0;
-    int *err = nullptr;
-    int qcand[3] = {0, 0, 0};     // the cost model's three best run-chunk counts, best first
-};
-
 // interior-kernel choice: variant 0 = one z plane per block, 1 = z-marching
 // over chunks of zchunk planes (0: the whole column)
 struct KCfg {
@@ -234,21 +183,6 @@ int k_stress_phy(int mode, const GridDev &g, const WaveDev &w, const float *lam,
 // or the driver entry point is missing.  Returns a cudaError_t.
 int k_make_wave_maps(const GridDev &g, const WaveDev &w, const float *lam, const float *mu, int *err_flag,
                      WaveMaps *maps);
-// The descriptors of the full-gridext stress kernel (variant 4), with the
-// run schedule cut into `chunks` chunks per tile (0: the cost model's
-// choice; maps->qcand lists its three best); maps->ok
-// stays false when the grid does not suit it (odd pml_num or nx, a tile
-// row of more than 512 threads or a halo row wider than 256 floats, the
-// driver entry point missing).  Returns a cudaError_t.
-int k_make_full_maps(const GridDev &g, const WaveDev &w, const float *lam, const float *mu, const float *vp,
-                     const float *bdt, float4 *const ax[3], float *psi, int *err_flag, int chunks,
-                     FullMaps *maps);
-// Stress update of every updated cell of gridext, interior and absorbing
-// layers in one launch (modes kFwd, kRtmFwd, kRev).
-int k_stress_full(int mode, const GridDev &g, const WaveDev &w, float dt, const float *wavelet, const StepState *st,
-                  int it_off, const FullMaps &maps, void *stream);
-// Velocity update of every updated cell of gridext (variant 4; vx, vy, vz)
-int k_vel_full(const GridDev &g, const WaveDev &w, float dt, const FullMaps &maps, void *stream);
 int k_vel_pml(const GridDev &g, const CpmlDev &c, const WaveDev &w, const float *bdt, const float *vp,
               const KCfg &kc, void *stream);
 int k_stress_pml(const GridDev &g, const CpmlDev &c, const WaveDev &w, const float *lam, const float *mu,
@@ -273,6 +207,8 @@ int k_image_stack(const GridDev &g, const ImageDev &shot, const StackDev &stack,
 // FP64 energy of the velocity and stress fields of w over gridphy, added into *out
 int k_wave_energy(const GridDev &g, const WaveDev &w, double *out, void *stream);
 int upload_coefficients(const float list[5][4], const float dc2[2]);
+// engine.cu: the staggered difference weights by half-order 1..4, zero past the order
+void staggered_taps(float list[5][4]);
 int k_count_nonfinite(const void *p, size_t n, int is_double, unsigned long long *out, void *stream);
 
 }  // namespace jv

@@ -82,9 +82,10 @@ typedef struct jv_options {
     int graph_steps;    /* time steps per captured graph (0 -> library default)  */
     size_t store_budget;/* max bytes of HBM for the boundary store (0 -> auto)   */
     int kernel_variant; /* stencil kernels: 0 one plane per block, 1 z-marching, 2 x-vectorised,
-                           3 as 2 with a TMA-fed z-marching stress update, 4 (default) as 3
-                           with the absorbing layers' stress update in the same TMA kernel
-                           (even pml_num and nx; other grids run variant 3's kernels);
+                           3 as 2 with a TMA-fed z-marching stress update, 4 (default) TMA-fed
+                           z-marching tile kernels for every stencil update, the absorbing
+                           layers in the same kernels (grids whose arrays reach 4 GB run
+                           variant 3's kernels);
                            -1: measured choice among 4, 3, 2, variant 4's run chunking,
                            the absorbing-layer register budget and the float4 kernels'
                            block shape on this grid at creation, kept per grid shape;
@@ -455,7 +456,9 @@ jv_status jv_rtm_reverse_end(jv_ctx *c);
  * directly (no graphs) and bracket each launch with CUDA events on the
  * context's stream; jv_profile_entry returns, for entry idx, the kernel
  * name, the summed device time and the launch count since profiling was
- * switched on (JV_EINVAL past the last entry).  The reference prints
+ * switched on (JV_EINVAL past the last entry).  A phase that another
+ * phase's kernel carries (an absorbing layer's update within gridext's) is
+ * listed with no launches.  The reference prints
  * per-shot times only (cuda_tic/cuda_toc, .jarvis_0_meta/.jarvis_0_math/
  * jarvis_2_device_math_bones.hpp:26-38). */
 jv_status jv_set_profiling(jv_ctx *c, int on);
