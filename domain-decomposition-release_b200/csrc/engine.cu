@@ -129,11 +129,14 @@ Engine::~Engine() {
     if (ev0_) cudaEventDestroy(ev0_);
     if (ev1_) cudaEventDestroy(ev1_);
     if (stream_) cudaStreamDestroy(stream_);
+    if (aux_) cudaStreamDestroy(aux_);
+    for (cudaEvent_t e : fev_)
+        if (e) cudaEventDestroy(e);
 }
 
 // ------------------------------------------------------------ layout helpers
 
-GridDev make_layout(const jv_grid &grid, size_t *field_elems) {
+GridDev make_layout(const jv_grid &grid, size_t *field_elems, bool tight) {
     GridDev g{};
     const int m = grid.pml;
     g.m = m;
@@ -143,7 +146,8 @@ GridDev make_layout(const jv_grid &grid, size_t *field_elems) {
     // 128-byte line, unless another offset (16-byte groups stay aligned)
     // lets the tile kernels' 32-column tiles, which start on such lines,
     // cover the rows with fewer tiles: four updates a migration step run over
-    // gridext, three over gridphy.
+    // gridext, three over gridphy.  Rows may grow by that where a field stays
+    // below 64 MB.
     auto tiles = [&](int xo) {
         const int f = (xo + 2) / 32 * 32, p = (xo + m) / 32 * 32;
         return 4 * ((xo + g.nx - 2 - f + 31) / 32) + 3 * ((xo + m + g.px - p + 31) / 32);
@@ -151,7 +155,10 @@ GridDev make_layout(const jv_grid &grid, size_t *field_elems) {
     g.xoff = (32 - (m % 32)) % 32;
     const int first = g.xoff;
     for (int xo = first % 4; xo < 32; xo += 4)
-        if (tiles(xo) < tiles(g.xoff)) g.xoff = xo;
+        if (tiles(xo) < tiles((int)g.xoff) &&
+            (round_up(xo + g.nx, 32) <= round_up(first + g.nx, 32) ||
+             (!tight && round_up(xo + g.nx, 32) * g.ny * g.nz < (16 << 20))))
+            g.xoff = xo;
     g.sy = round_up(g.xoff + g.nx, 32);
     g.sz = g.sy * g.ny;
     g.dx = grid.dx; g.dy = grid.dy; g.dz = grid.dz;
@@ -851,11 +858,33 @@ Status Engine::check_finite(const char *after) {
         if (check_finite_) JV_TRY(check_finite(name));                      \
     } while (0)
 
+// While a step is captured with two branches: what follows on `after` waits
+// for what is on `before` (event ev).  Nothing when there is one branch.
+Status Engine::order(int ev, cudaStream_t before, cudaStream_t after) {
+    if (!fork_) return Status{};
+    JV_CU(cudaEventRecord(fev_[ev], before));
+    JV_CU(cudaStreamWaitEvent(after, fev_[ev], 0));
+    return Status{};
+}
+
 // The kernels of one time step of `kind`.  They read the time step as
 // st_->it + off; advance == true ends the step with st_->it += direction.
-Status Engine::launch_step(int kind, int off, bool advance) {
+// In a captured chunk of steps (first, last: its ends) with the tile
+// kernels, phases on disjoint arrays form a second branch, so that one
+// fills the SMs that the other's last blocks leave and small grids run two
+// kernels at once:
+//   modelling    the receivers' record (reads v) beside the stress update
+//   RTM forward  the velocity boxes' pack beside the stress update, the
+//                stress boxes' beside the next velocity update
+//   reverse      the reconstruction (stress, boundary boxes, velocity) beside
+//                the receiver wavefield's injection and velocity update;
+//                imaging joins them; the receiver stress update then runs
+//                beside the next step's reconstruction
+Status Engine::launch_step(int kind, int off, bool advance, bool first, bool last) {
     cur_kind_ = kind;
     void *s = (void *)stream_;
+    const cudaStream_t side = fork_ ? aux_ : stream_;
+    void *s2 = (void *)side;
     const float dt = dt_;
     const int rw = opt_.rec_width;
     switch (kind) {
@@ -863,26 +892,35 @@ Status Engine::launch_step(int kind, int off, bool advance) {
         if (tiles_) {
             if (wide_) folded("vel_pml"), folded("vel_phy_fwd");
             JV_L(wide_ ? "vel_tile_fwd" : "vel_fz_fwd", k_vel_tile(kFwd, g_, F_, bdt_, vp_, dt, rw, tileF_, s));
+            JV_TRY(order(0, stream_, side));
             JV_L("stress_fz_fwd",
                  k_stress_tile(kFwd, g_, F_, lam_, mu_, vp_, dt, rw, wavelet_, st_, off, tileF_, s));
+            JV_L("record", k_record(F_, rec_d_, nrec_, nt_, st_, off, s2));
+            JV_TRY(order(1, side, stream_));
         } else {
             JV_L("vel_pml", k_vel_pml(g_, cpF_, F_, bdt_, vp_, kc_, s));
             JV_L("vel_phy_fwd", k_vel_phy(kFwd, g_, F_, bdt_, dt, rw, nullptr, nullptr, kc_, s));
             JV_L("stress_pml", k_stress_pml(g_, cpF_, F_, lam_, mu_, vp_, 0, kc_, s));
             JV_L("stress_phy_fwd",
                  k_stress_phy(kFwd, g_, F_, lam_, mu_, dt, rw, wavelet_, st_, off, kc_, s, &mapsF_));
+            JV_L("record", k_record(F_, rec_d_, nrec_, nt_, st_, off, s));
         }
-        JV_L("record", k_record(F_, rec_d_, nrec_, nt_, st_, off, s));
         if (advance) JV_L("step_advance", k_step_advance(st_, +1, s));
         break;
     case kStepRtmFwd:
         if (tiles_) {
             if (wide_) folded("vel_pml"), folded("vel_phy_rtmfwd");
             JV_L(wide_ ? "vel_tile_rtmfwd" : "vel_fz_rtmfwd", k_vel_tile(kRtmFwd, g_, F_, bdt_, vp_, dt, rw, tileF_, s));
-            // the boundary boxes lie in the absorbing layers: pack them after their update
+            // the boundary boxes lie in the absorbing layers: packed after their update
+            JV_TRY(order(0, stream_, side));
+            if (!first) JV_TRY(order(2, side, stream_));  // the step before's stress boxes are packed
+            JV_L("vowr_pack", k_vowr(g_, F_, vowr_, st_, off, 1, 1, s2));
             JV_L("stress_fz_rtmfwd",
                  k_stress_tile(kRtmFwd, g_, F_, lam_, mu_, vp_, dt, rw, wavelet_, st_, off, tileF_, s));
-            JV_L("vowr_pack", k_vowr(g_, F_, vowr_, st_, off, 1, 0, s));
+            JV_TRY(order(1, side, stream_));
+            JV_TRY(order(0, stream_, side));
+            JV_L("vowr_pack", k_vowr(g_, F_, vowr_, st_, off, 1, 2, s2));
+            if (last) JV_TRY(order(2, side, stream_));
         } else {
             JV_L("vel_pml", k_vel_pml(g_, cpF_, F_, bdt_, vp_, kc_, s));
             JV_L("vel_phy_rtmfwd", k_vel_phy(kRtmFwd, g_, F_, bdt_, dt, rw, nullptr, nullptr, kc_, s));
@@ -895,35 +933,39 @@ Status Engine::launch_step(int kind, int off, bool advance) {
         break;
     case kStepRtmRev:
         // UPDATE 1: source subtraction (fused) + backward stress, receiver
-        // injection + reverse velocity, stress boundary layers of step it-1
-        JV_L("inject_rec", k_inject_rec(R_, rec_d_, nrec_, nt_, st_, off, s));
+        // injection + reverse velocity, stress boundary layers of step it-1;
+        // UPDATE 2: backward velocity with the imaging condition fused,
+        // reverse stress, velocity boundary layers of step it-1
         if (tiles_) {
+            if (first) JV_TRY(order(0, stream_, side));
             JV_L("stress_tile_bwd",
-                 k_stress_tile(kBwd, g_, F_, lam_, mu_, vp_, -dt, rw, wavelet_, st_, off, tileFB_, s));
+                 k_stress_tile(kBwd, g_, F_, lam_, mu_, vp_, -dt, rw, wavelet_, st_, off, tileFB_, s2));
+            JV_L("vowr_unpack", k_vowr(g_, F_, vowr_, st_, off - 1, 0, 2, s2));
+            JV_L("vel_tile_bwd", k_vel_tile(kBwd, g_, F_, bdt_, vp_, -dt, rw, tileFB_, s2));
+            // outside gridphy, which the imaging does not read
+            JV_L("vowr_unpack", k_vowr(g_, F_, vowr_, st_, off - 1, 0, 1, s2));
             // the receiver side's velocities, absorbing layers included; its
             // P-wave velocities follow in the imaging kernel
+            JV_L("inject_rec", k_inject_rec(R_, rec_d_, nrec_, nt_, st_, off, s));
             folded("vel_pml"), folded("vel_phy_rev");
             JV_L("vel_tile_rev", k_vel_tile(kRev, g_, R_, bdt_, vp_, dt, rw, tileR_, s));
+            JV_TRY(order(1, side, stream_));
+            JV_L("pvel_image", k_pvel_tile(g_, &F_, &tileFB_, R_, tileRB_, true, bdt_, rw, &shot_img_, s));
+            if (!last) JV_TRY(order(0, stream_, side));
+            JV_L("stress_fz_rev", k_stress_tile(kRev, g_, R_, lam_, mu_, vp_, dt, rw, wavelet_, st_, off, tileR_, s));
         } else {
+            JV_L("inject_rec", k_inject_rec(R_, rec_d_, nrec_, nt_, st_, off, s));
             JV_L("stress_phy_bwd",
                  k_stress_phy(kBwd, g_, F_, lam_, mu_, -dt, rw, wavelet_, st_, off, kc_, s, &mapsF_));
             JV_L("vel_pml", k_vel_pml(g_, cpR_, R_, bdt_, vp_, kc_, s));
             JV_L("vel_phy_rev", k_vel_phy(kRev, g_, R_, bdt_, dt, rw, nullptr, nullptr, kc_, s));
-        }
-        JV_L("vowr_unpack", k_vowr(g_, F_, vowr_, st_, off - 1, 0, 2, s));
-        // UPDATE 2: backward velocity with the imaging condition fused,
-        // reverse stress, velocity boundary layers of step it-1
-        if (tiles_) {
-            JV_L("vel_tile_bwd", k_vel_tile(kBwd, g_, F_, bdt_, vp_, dt, rw, tileFB_, s));
-            JV_L("pvel_image", k_pvel_tile(g_, &F_, &tileFB_, R_, tileRB_, true, bdt_, rw, &shot_img_, s));
-            JV_L("stress_fz_rev", k_stress_tile(kRev, g_, R_, lam_, mu_, vp_, dt, rw, wavelet_, st_, off, tileR_, s));
-        } else {
+            JV_L("vowr_unpack", k_vowr(g_, F_, vowr_, st_, off - 1, 0, 2, s));
             JV_L("vel_phy_bwd_image", k_vel_phy(kBwd, g_, F_, bdt_, -dt, rw, &R_, &shot_img_, kc_, s));
             JV_L("stress_pml_sau", k_stress_pml(g_, cpR_, R_, lam_, mu_, vp_, 1, kc_, s));
             JV_L("stress_phy_rev",
                  k_stress_phy(kRev, g_, R_, lam_, mu_, dt, rw, wavelet_, st_, off, kc_, s, &mapsR_));
+            JV_L("vowr_unpack", k_vowr(g_, F_, vowr_, st_, off - 1, 0, 1, s));
         }
-        JV_L("vowr_unpack", k_vowr(g_, F_, vowr_, st_, off - 1, 0, 1, s));
         if (advance) JV_L("step_advance", k_step_advance(st_, -1, s));
         break;
     default: return bad(JV_EINVAL, "unknown step kind");
@@ -949,13 +991,19 @@ Status Engine::run_loop(int kind, int nsteps) {
             *ex = it->second;
             return Status{};
         }
+        if (tiles_ && !aux_) {
+            for (cudaEvent_t &e : fev_) JV_CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            JV_CU(cudaStreamCreateWithFlags(&aux_, cudaStreamNonBlocking));
+        }
         cudaGraph_t gr;
         JV_CU(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
         Status st;
         // one capture of `steps` time steps: step i reads st_->it + dir*i,
         // and one advance by dir*steps ends the chunk
         const int dir = kind == kStepRtmRev ? -1 : +1;
-        for (int i = 0; i < steps && st; i++) st = launch_step(kind, dir * i, false);
+        fork_ = tiles_;
+        for (int i = 0; i < steps && st; i++) st = launch_step(kind, dir * i, false, i == 0, i == steps - 1);
+        fork_ = false;
         if (st) {
             int ek = k_step_advance(st_, dir * steps, stream_);
             if (ek != 0) st = bad(JV_ECUDA, std::string("step_advance: ") + cudaGetErrorString((cudaError_t)ek));

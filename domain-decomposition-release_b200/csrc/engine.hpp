@@ -40,8 +40,8 @@ jv_status rtm_self_modelled(jv_ctx *c, int shot);
 // Pitched gridext layout of a gridphy + pml problem (elem = base + xoff +
 // i + sy*j + sz*k, first gridphy column 16-byte aligned); *field_elems =
 // floats of one field array (gridext plus tail slack for the aligned
-// x groups of the absorbing-layer kernels).
-GridDev make_layout(const jv_grid &grid, size_t *field_elems);
+// x groups of the absorbing-layer kernels); tight: rows as short as can be.
+GridDev make_layout(const jv_grid &grid, size_t *field_elems, bool tight = false);
 // The six CPML slabs (FD/fdtd3d_0_base_module/fdtd3d_base_6_pml_meat.hpp:29-94)
 // with their launch shapes and memory-variable arena offsets; *psi_total =
 // floats of one wavefield's memory-variable arena.  dt, ax and psi are
@@ -122,7 +122,8 @@ class Engine {
     Status upload_model(const float *vp, const float *vs, const float *rho);
     Status check_shot(int shot, long long *src) const;
     Status run_loop(int kind, int nsteps);
-    Status launch_step(int kind, int off, bool advance);
+    Status launch_step(int kind, int off, bool advance, bool first = true, bool last = true);
+    Status order(int ev, cudaStream_t before, cudaStream_t after);
     Status autotune(bool neutral);
     Status make_tiles();
 
@@ -157,6 +158,12 @@ class Engine {
     int nt_ = 0;
     int dev_ = 0;
     cudaStream_t stream_ = nullptr;
+    // a second branch of the captured time loops: while fork_ is set (during
+    // capture only) the phases of a step that do not touch one another's
+    // arrays are recorded on aux_ beside stream_
+    cudaStream_t aux_ = nullptr;
+    cudaEvent_t fev_[3] = {nullptr, nullptr, nullptr};
+    bool fork_ = false;
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
     double last_ms_ = 0.0;
 

@@ -1601,13 +1601,13 @@ __global__ void __launch_bounds__(256) vowr(GridDev g, const __grid_constant__ W
 // cleared for the next step.
 __global__ void __launch_bounds__(256) vowr_amax(GridDev g, const __grid_constant__ WaveDev w,
                                                  const __grid_constant__ VowrDev v,
-                                                 const StepState *__restrict__ st, int slot_shift) {
+                                                 const StepState *__restrict__ st, int slot_shift, int b0) {
     const int slot = st->it + slot_shift;
     if (slot < 0 || slot >= v.nslot) return;
     unsigned *cur = v.amax + (slot & 1) * v.nseg, *nxt = v.amax + ((slot + 1) & 1) * v.nseg;
     if (blockIdx.x == 0)
         for (int q = threadIdx.x; q < v.nseg; q += blockDim.x) nxt[q] = 0u;
-    const int b = (int)blockIdx.x;
+    const int b = b0 + (int)blockIdx.x;
     const int sg = vowr_box(v, b);
     const SegDev &S = v.seg[sg];
     const int e = (b - (int)S.nblk_first) * 256 + (int)threadIdx.x;
@@ -2087,10 +2087,7 @@ int k_vowr(const GridDev &g, const WaveDev &w, const VowrDev &v, const StepState
         vowr<<<(unsigned)(b1 - b0), 256, 0, s>>>(g, w, v, st, slot_shift, pack, b0);
         return cerr();
     }
-    if (pack) {
-        if (b0 != 0 || b1 != v.all_blocks) return (int)cudaErrorInvalidValue;  // a step's boxes pack together
-        vowr_amax<<<(unsigned)v.all_blocks, 256, 0, s>>>(g, w, v, st, slot_shift);
-    }
+    if (pack) vowr_amax<<<(unsigned)(b1 - b0), 256, 0, s>>>(g, w, v, st, slot_shift, b0);
     if (v.prec == kStoreBF16) vowr16<kStoreBF16><<<(unsigned)(b1 - b0), 256, 0, s>>>(g, w, v, st, slot_shift, pack, b0);
     else vowr16<kStoreFP16><<<(unsigned)(b1 - b0), 256, 0, s>>>(g, w, v, st, slot_shift, pack, b0);
     return cerr();

@@ -137,14 +137,12 @@ extern "C" jv_status jv_forward_noalloc(const jv_grid *grid, const float *d_vp, 
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return fail(JV_ECUDA, std::string("cudaGetDevice: ") + cudaGetErrorString(e));
 
-    // layout and CPML slabs: the same as the context path
+    // layout and kernels: the same as the context path's
     const int m = grid->pml;
     size_t fe = 0;
-    const GridDev g = make_layout(*grid, &fe);
+    const GridDev g = make_layout(*grid, &fe, true);
     const size_t guard = 32;
-    long long psi_total = 0;
-    CpmlDev cp = make_pml_slabs(g, 1, &psi_total);
-    cp.dt = dt;
+    const long long psi_total = tile_psi_floats(g);
 
     // receivers inside gridphy, in input order (as jv_set_geometry keeps them)
     const float rx = (float)(g.px - 1) * g.dx, ry = (float)(g.py - 1) * g.dy, rz = (float)(g.pz - 1) * g.dz;
@@ -173,8 +171,9 @@ extern "C" jv_status jv_forward_noalloc(const jv_grid *grid, const float *d_vp, 
     for (int a = 0; a < 3; a++) tabs[a] = cv.take<float4>((size_t)(a == 0 ? g.nx : a == 1 ? g.ny : g.nz));
     float *wavelet = cv.take<float>((size_t)nt);
     StepState *state = cv.take<StepState>(1);
+    int *err_d = cv.take<int>(1);
     long long *rec_d = cv.take<long long>(rec.size() + 1);
-    if (!model || !wave || (psi_total && !psi) || !tabs[0] || !tabs[1] || !tabs[2] || !wavelet || !state || !rec_d)
+    if (!model || !wave || (psi_total && !psi) || !tabs[0] || !tabs[1] || !tabs[2] || !wavelet || !state || !err_d || !rec_d)
         return fail(JV_EINVAL, "problem needs more than the " + std::to_string(kNoAllocScratchBytes >> 20) +
                                    " MiB no-allocation scratch; use jv_create/jv_forward");
     if (fe >= ((size_t)1 << 31)) return fail(JV_EINVAL, "grid too large");
@@ -213,26 +212,32 @@ extern "C" jv_status jv_forward_noalloc(const jv_grid *grid, const float *d_vp, 
     // the previous call left its state here: clear what must start at zero
     NA_CK(cudaMemsetAsync(model, 0, (4 * fe + guard) * sizeof(float), s));
     NA_CK(cudaMemsetAsync(wave, 0, (9 * fe + guard) * sizeof(float), s));
-    if (psi_total) NA_CK(cudaMemsetAsync(psi, 0, (size_t)psi_total * sizeof(float), s));
+    NA_CK(cudaMemsetAsync(psi, 0, (size_t)psi_total * sizeof(float), s));
+    NA_CK(cudaMemsetAsync(err_d, 0, sizeof(int), s));
 
     float *mb = model + guard;
     float *vp = mb, *bdt = mb + fe, *lam = mb + 2 * fe, *mu = mb + 3 * fe;
     NA_CK(k_model_prep(g, d_vp, d_vs, d_rho, dt, vp, bdt, lam, mu, s));
     WaveDev w{};
     for (int f = 0; f < 9; f++) w.f[f] = wave + guard + f * fe;
-    for (int a = 0; a < 3; a++) cp.ax[a] = tabs[a];
-    cp.psi = psi;
-    KCfg kc;
-    kc.variant = 2;
-    for (int it = 0; it < nt; it++) {
-        NA_CK(k_vel_pml(g, cp, w, bdt, vp, kc, s));
-        NA_CK(k_vel_phy(kFwd, g, w, bdt, dt, 1, nullptr, nullptr, kc, s));
-        NA_CK(k_stress_pml(g, cp, w, lam, mu, vp, 0, kc, s));
-        NA_CK(k_stress_phy(kFwd, g, w, lam, mu, dt, 1, wavelet, state, 0, kc, s));
-        NA_CK(k_record(w, rec_d, (int)rec.size(), nt, state, 0, s));
-        NA_CK(k_step_advance(state, +1, s));
+    TileMaps tm;
+    NA_CK(k_make_tile_maps(g, w, false, tabs, psi, err_d, 0, &tm));
+    if (!tm.ok) {
+        (void)cudaStreamSynchronize(s);
+        return fail(JV_ENOTSUP, "tensor-map encoding is not available from this driver");
     }
+    // three launches a step, each told its step: the caller's stream is fed
+    // from here, and with six (the split kernels and a counter) the host was
+    // what a small model waited for (45 us a step at 32 x 28 x 24)
+    for (int it = 0; it < nt; it++) {
+        NA_CK(k_vel_tile(kFwd, g, w, bdt, vp, dt, 1, tm, s));
+        NA_CK(k_stress_tile(kFwd, g, w, lam, mu, vp, dt, 1, wavelet, state, it, tm, s));
+        NA_CK(k_record(w, rec_d, (int)rec.size(), nt, state, it, s));
+    }
+    int err_h = 0;
+    NA_CK(cudaMemcpyAsync(&err_h, err_d, sizeof(int), cudaMemcpyDeviceToHost, s));
     NA_CK(cudaStreamSynchronize(s));
+    if (err_h) return fail(JV_ETIMEOUT, "a shared-memory tile of a tile kernel did not arrive in time");
 #undef NA_CK
     jv::set_last_error("");
     return JV_OK;
