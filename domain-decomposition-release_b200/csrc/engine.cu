@@ -397,11 +397,10 @@ Status Engine::create(const jv_grid &grid, const float *vp, const float *vs, con
 // apply, with the cost model's three best run chunkings (unless run_chunks
 // fixes one), variant 3 where its stress kernel applies, variant 2 -- and,
 // for the variants with separate absorbing-layer kernels, their register
-// budget (3 or 4 blocks per SM).  Then, unless tile_gx / tile_gy were
-// given, the float4 kernels' block shape: the default number of blocks per
+// budget (3 or 4 blocks per SM).  Then, for a choice that runs them and
+// unless tile_gx / tile_gy were given, the float4 kernels' block shape: the default number of blocks per
 // gridphy row and one fewer or one more, timed on the reverse loop's
-// float4 velocity update and the backward stress update (the forward step
-// of a one-tile grid does not run them).  The fastest wins; the choice is
+// float4 velocity update and the backward stress update.  The fastest wins; the choice is
 // kept per grid shape and device for the contexts that follow.
 Status Engine::autotune(bool neutral) {
     struct Cand {
