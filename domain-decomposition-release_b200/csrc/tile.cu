@@ -37,6 +37,7 @@
 #include <cstring>
 #include <utility>
 
+#include "damping.hpp"
 #include "jv_internal.hpp"
 #include "tile.hpp"
 #include "tma.cuh"
@@ -196,29 +197,17 @@ __device__ __forceinline__ int rim_order(int p, int np, int w) {
 
 // ------------------------------------------------ absorbing layers
 //
-// Damping of one node: d = vp K, b = exp(-(d + alpha) dt), a = d (b - 1) /
-// (d + alpha); K and alpha of the pair's two cells, both zero for a cell that
-// does not absorb (a = 0 then).  The layer's response to slow fields is 1 +
-// a / (1 - b) = alpha / (d + alpha), a small number at the outer cells, so a
-// is formed as (b - 1) (1 - alpha / (d + alpha)) from the rounded b: the
-// quotient's error then counts against alpha / (d + alpha) and not against
-// one, and a hardware estimate with one Newton step will do (no branch of a
-// division).
-__device__ __forceinline__ float rcp_estimate(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
+// damping of a pair; a cell that does not absorb has K and alpha zero
 __device__ __forceinline__ void damping(f2 vp, f2 K, f2 alpha, f2 dt, f2 &A, f2 &B) {
-    const f2 d = mul2(vp, K), e = add2(d, alpha), minus = dup(-1.f);
-    float u, v, s, t;
-    up(mul2(mul2(e, minus), dt), s, t);
-    B = pk(expf(s), expf(t));
-    up(e, u, v);
-    f2 r = pk(rcp_estimate(u == 0.f ? 1.f : u), rcp_estimate(v == 0.f ? 1.f : v));
-    r = fma2(r, fma2(mul2(e, minus), r, dup(1.f)), r);
-    const f2 w = add2(B, minus);
-    A = fma2(mul2(w, minus), mul2(alpha, r), w);
+    float v0, v1, k0, k1, l0, l1, t0, t1, a0, a1, b0, b1;
+    up(vp, v0, v1);
+    up(K, k0, k1);
+    up(alpha, l0, l1);
+    up(dt, t0, t1);
+    damping_ab(v0, k0, l0, t0, a0, b0);
+    damping_ab(v1, k1, l1, t1, a1, b1);
+    A = pk(a0, a1);
+    B = pk(b0, b1);
 }
 
 // the thread's place in its tile
