@@ -130,44 +130,48 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // ------------------------------------------------ differences
 //
 // Dp f = sum_q c_q (f[i+(q+1)s] - f[i-qs]);  Dm f = sum_q c_q (f[i+qs] - f[i-(q+1)s])
+// in cells of the grid (callers multiply by 1 / spacing).  Single cells of an
+// image are differences of nearly equal numbers, where one rounding more or
+// another order shows at 1 %; so the rounding here and in the sums of
+// differences is fixed, and a test pins it bit for bit.  gridphy sums its four
+// terms from q = 0 on, an absorbing layer its two from q = 1 on: with AB
+// (kernels that run in layers) the term q = 0 has a weight at either end of
+// the chain, C[0] and C[4], one of them zero.
 
 // along x, at the pair F[0..1] of a row in shared memory; C: the weights of
 // the two cells; mid: the pair itself
-template <bool PLUS>
-__device__ __forceinline__ f2 diff_x(const float *F, const f2 C[4], f2 rd, f2 &mid) {
+template <bool PLUS, bool AB>
+__device__ __forceinline__ f2 diff_x(const float *F, const f2 *C, f2 &mid) {
     float e[10];
     mid = at2(F);
 #pragma unroll
     for (int j = 0; j < 5; j++) up(j == 2 ? mid : at2(F - 4 + 2 * j), e[2 * j], e[2 * j + 1]);
     constexpr int o = PLUS ? 5 : 4;
-    f2 t = 0;
+    const f2 d0 = pk(e[o] - e[o - 1], e[o + 1] - e[o]);
+    f2 t = mul2(C[0], d0);
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const f2 d = pk(e[o + q] - e[o - 1 - q], e[o + 1 + q] - e[o - q]);
-        t = q == 0 ? mul2(C[0], d) : fma2(C[q], d, t);
-    }
-    return mul2(t, rd);
+    for (int q = 1; q < 4; q++) t = fma2(C[q], pk(e[o + q] - e[o - 1 - q], e[o + 1 + q] - e[o - q]), t);
+    return AB ? fma2(C[4], d0, t) : t;
 }
 // along y: rows PITCH floats apart
-template <bool PLUS, int PITCH>
-__device__ __forceinline__ f2 diff_y(const float *F, const f2 C[4], f2 rd) {
+template <bool PLUS, bool AB, int PITCH>
+__device__ __forceinline__ f2 diff_y(const float *F, const f2 *C) {
     constexpr int o = PLUS ? 1 : 0;
-    f2 t = 0;
+    const f2 d0 = sub2(at2(F + o * PITCH), at2(F - (1 - o) * PITCH));
+    f2 t = mul2(C[0], d0);
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const f2 d = sub2(at2(F + (q + o) * PITCH), at2(F - (q + 1 - o) * PITCH));
-        t = q == 0 ? mul2(C[0], d) : fma2(C[q], d, t);
-    }
-    return mul2(t, rd);
+    for (int q = 1; q < 4; q++) t = fma2(C[q], sub2(at2(F + (q + o) * PITCH), at2(F - (q + 1 - o) * PITCH)), t);
+    return AB ? fma2(C[4], d0, t) : t;
 }
 // along z: mid is this plane's pair, F the field's place in a buffer and off
 // the buffers of this plane and the four above; w the pairs of the planes
 // below, oldest first (three of them with PLUS, else four), which move on
-template <bool PLUS>
-__device__ __forceinline__ f2 diff_z(const float *F, const int off[5], f2 mid, f2 *w, const f2 C[4], f2 rd) {
-    f2 t;
+template <bool PLUS, bool AB>
+__device__ __forceinline__ f2 diff_z(const float *F, const int off[5], f2 mid, f2 *w, const f2 *C) {
+    f2 d0, t;
     if (PLUS) {
-        t = mul2(C[0], sub2(at2(F + off[1]), mid));
+        d0 = sub2(at2(F + off[1]), mid);
+        t = mul2(C[0], d0);
         t = fma2(C[1], sub2(at2(F + off[2]), w[2]), t);
         t = fma2(C[2], sub2(at2(F + off[3]), w[1]), t);
         t = fma2(C[3], sub2(at2(F + off[4]), w[0]), t);
@@ -175,7 +179,8 @@ __device__ __forceinline__ f2 diff_z(const float *F, const int off[5], f2 mid, f
         w[1] = w[2];
         w[2] = mid;
     } else {
-        t = mul2(C[0], sub2(mid, w[3]));
+        d0 = sub2(mid, w[3]);
+        t = mul2(C[0], d0);
         t = fma2(C[1], sub2(at2(F + off[1]), w[2]), t);
         t = fma2(C[2], sub2(at2(F + off[2]), w[1]), t);
         t = fma2(C[3], sub2(at2(F + off[3]), w[0]), t);
@@ -184,8 +189,27 @@ __device__ __forceinline__ f2 diff_z(const float *F, const int off[5], f2 mid, f
         w[2] = w[3];
         w[3] = mid;
     }
-    return mul2(t, rd);
+    return AB ? fma2(C[4], d0, t) : t;
 }
+// weights of the two cells of a pair; p0, p1: whether they lie in gridphy
+__device__ __forceinline__ void set_weights(f2 C[5], bool p0, bool p1, const TileGeo &q) {
+    C[0] = pk(p0 ? q.taps[4][0] : 0.f, p1 ? q.taps[4][0] : 0.f);
+    C[4] = pk(p0 ? 0.f : q.taps[2][0], p1 ? 0.f : q.taps[2][0]);
+#pragma unroll
+    for (int j = 1; j < 4; j++) C[j] = pk(p0 ? q.taps[4][j] : q.taps[2][j], p1 ? q.taps[4][j] : q.taps[2][j]);
+}
+// Adding a difference t to another one: in gridphy one fused multiply-add, t r
+// + sum with r = 1 / spacing; in a layer t r is rounded first, for its memory
+// variable, and then added.  (t S) R + sum serves a pair with a cell of
+// either kind: S = 1 and R = r, or S = r and R = 1.  Pairs of gridphy, most of
+// them, take the fused form from a branch of their own: with S and R kept in
+// registers for all pairs the stress update ran at 275 against 264 us
+// (200^3 + 20), short of registers.
+struct Join {
+    f2 S, R;
+    __device__ __forceinline__ Join(bool p0, bool p1, float r)
+        : S(pk(p0 ? 1.f : r, p1 ? 1.f : r)), R(pk(p0 ? r : 1.f, p1 ? r : 1.f)) {}
+};
 
 // Order of one axis in the rtm_backward rim: within 4 cells of a gridphy
 // face the order drops to e+1 (e = distance to the face) but never below
@@ -478,8 +502,8 @@ __global__ void __launch_bounds__(kThreads, 2)
         psi.fetch(g, q, vpm, 4u * (uint32_t)t.i0, t.z0, 0, live, xab, yab, zabs(t.z0));
         copy_commit();
     }
-    int zclass = -1;  // whether the weights in cx are those of a plane of gridphy
-    f2 cx[4];
+    int zclass = -1;  // whether the weights are those of a plane of gridphy
+    f2 cx[5];
     if (!kCp) {
         const int o0 = rim_order(min(max(t.x - m, 0), g.px - 1), g.px, rec_w);
         const int o1 = rim_order(min(max(t.x + 1 - m, 0), g.px - 1), g.px, rec_w);
@@ -517,15 +541,13 @@ __global__ void __launch_bounds__(kThreads, 2)
         if (pf && k + kAhead < t.n) prefetch_line(pf + (long long)k * sz);
         ok = rd.wait();
         if (!ok) break;
-        const bool zph = !zabs(z);
+        const bool zph = !zabs(z), p0 = ph0 && yph && zph, p1 = ph1 && yph && zph;
+        const bool ab = kCp && !(p0 && p1);  // a cell of the pair lies in a layer
         f2 vp = 0;
         if (kCp) {
             if (zclass != (int)zph) {
                 zclass = zph;
-                const bool p = yph && zph;
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    cx[j] = pk(p && ph0 ? q.taps[4][j] : q.taps[2][j], p && ph1 ? q.taps[4][j] : q.taps[2][j]);
+                set_weights(cx, p0, p1, q);
             }
             copy_wait1();
             __syncwarp();
@@ -534,35 +556,50 @@ __global__ void __launch_bounds__(kThreads, 2)
         const float *F = S + rd.off[0];
         // normal differences Nx = d vx/dx, ...; shear sums Sxy = d vy/dx + d vx/dy, ...
         f2 mx, my, mz;
-        f2 Nx = diff_x<false>(F, cx, rdx, mx);
-        f2 Sxy = diff_x<true>(F + kSField, cx, rdx, my);
-        f2 Sxz = diff_x<true>(F + 2 * kSField, cx, rdx, mz);
-        if (kCp && xab)
-            absorb_x<false>(psi.at(k & 1, 1), q.psx[1], psi.ix(z), psi.tab[t.c], psi.tab[t.c + 1], vp, dt2, Nx, Sxy, Sxz);
+        f2 Nx = mul2(diff_x<false, kCp>(F, cx, mx), rdx);
+        f2 Sxy = diff_x<true, kCp>(F + kSField, cx, my);
+        f2 Sxz = diff_x<true, kCp>(F + 2 * kSField, cx, mz);
+        if (ab) {
+            const Join jx(p0, p1, 1.0f / g.dx);
+            Sxy = mul2(Sxy, jx.S);
+            Sxz = mul2(Sxz, jx.S);
+            if (xab)
+                absorb_x<false>(psi.at(k & 1, 1), q.psx[1], psi.ix(z), psi.tab[t.c], psi.tab[t.c + 1], vp, dt2, Nx, Sxy, Sxz);
+        }
         f2 Ny, Syz;
         {
-            f2 cy[4];
+            f2 cy[5];
 #pragma unroll
-            for (int j = 0; j < 4; j++) cy[j] = kCp ? cx[j] : rows[rim_order(t.y - m, g.py, rec_w)][j];
-            Ny = diff_y<false, kPW>(F + kSField, cy, rdy);
-            f2 a = diff_y<true, kPW>(F, cy, rdy);
-            Syz = diff_y<true, kPW>(F + 2 * kSField, cy, rdy);
-            if (kCp && yab)
-                absorb_yz<false>(psi.at(k & 1, 4), q.psy[1], psi.iy(z), psi.tab[kTX + t.r], vp, dt2, Ny, a, Syz);
-            Sxy = add2(Sxy, a);
+            for (int j = 0; j < (kCp ? 5 : 4); j++) cy[j] = kCp ? cx[j] : rows[rim_order(t.y - m, g.py, rec_w)][j];
+            Ny = mul2(diff_y<false, kCp, kPW>(F + kSField, cy), rdy);
+            f2 a = mul2(diff_y<true, kCp, kPW>(F, cy), rdy);
+            Syz = diff_y<true, kCp, kPW>(F + 2 * kSField, cy);
+            if (ab) {
+                Syz = mul2(Syz, Join(p0, p1, 1.0f / g.dy).S);
+                if (yab)
+                    absorb_yz<false>(psi.at(k & 1, 4), q.psy[1], psi.iy(z), psi.tab[kTX + t.r], vp, dt2, Ny, a, Syz);
+                Sxy = fma2(Sxy, Join(p0, p1, 1.0f / g.dx).R, a);
+            } else {
+                Sxy = fma2(Sxy, rdx, a);
+            }
         }
-        f2 cz[4];
+        f2 cz[5];
 #pragma unroll
-        for (int j = 0; j < 4; j++) cz[j] = kCp ? cx[j] : rows[rim_order(z - m, g.pz, rec_w)][j];
-        f2 Nz = diff_z<false>(S + 2 * kSField, rd.off, mz, wz, cz, rdz);
-        f2 a = diff_z<true>(S, rd.off, mx, wx, cz, rdz);
-        f2 b = diff_z<true>(S + kSField, rd.off, my, wy, cz, rdz);
+        for (int j = 0; j < (kCp ? 5 : 4); j++) cz[j] = kCp ? cx[j] : rows[rim_order(z - m, g.pz, rec_w)][j];
+        f2 Nz = mul2(diff_z<false, kCp>(S + 2 * kSField, rd.off, mz, wz, cz), rdz);
+        f2 a = mul2(diff_z<true, kCp>(S, rd.off, mx, wx, cz), rdz);
+        f2 b = mul2(diff_z<true, kCp>(S + kSField, rd.off, my, wy, cz), rdz);
         rd.release();
         rd.next(AF);
-        if (kCp && live && !zph)
-            absorb_yz<false>(psi.at(k & 1, 7), q.psz[1], psi.iz(g, z), psi.zrow(k & 1), vp, dt2, Nz, a, b);
-        Sxz = add2(Sxz, a);
-        Syz = add2(Syz, b);
+        if (ab) {
+            if (live && !zph)
+                absorb_yz<false>(psi.at(k & 1, 7), q.psz[1], psi.iz(g, z), psi.zrow(k & 1), vp, dt2, Nz, a, b);
+            Sxz = fma2(Sxz, Join(p0, p1, 1.0f / g.dx).R, a);
+            Syz = fma2(Syz, Join(p0, p1, 1.0f / g.dy).R, b);
+        } else {
+            Sxz = fma2(Sxz, rdx, a);
+            Syz = fma2(Syz, rdy, b);
+        }
         if (MODE != kRev && k == src_k) {
             // explosive source, applied before the stress update of step it
             // (FD/fdtd3d_2_phy_mpi_module/fdtd3d_phy_mpi_3_stress_kernel.hpp:1308-1364)
@@ -574,9 +611,9 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
         const f2 l2m = fma2(pm, dup(2.0f), pl), dm = mul2(dt2, pm);
         f2 v[kSau ? 7 : 6];
-        v[0] = fma2(dt2, fma2(pl, Nz, fma2(pl, Ny, mul2(l2m, Nx))), ps[0]);
-        v[1] = fma2(dt2, fma2(pl, Nz, fma2(l2m, Ny, mul2(pl, Nx))), ps[1]);
-        v[2] = fma2(dt2, fma2(l2m, Nz, fma2(pl, Ny, mul2(pl, Nx))), ps[2]);
+        v[0] = fma2(dt2, fma2(pl, Nz, fma2(l2m, Nx, mul2(pl, Ny))), ps[0]);
+        v[1] = fma2(dt2, fma2(pl, Nz, fma2(pl, Nx, mul2(l2m, Ny))), ps[1]);
+        v[2] = fma2(dt2, fma2(l2m, Nz, fma2(pl, Nx, mul2(pl, Ny))), ps[2]);
         v[3] = fma2(dm, Sxy, ps[3]);
         v[4] = fma2(dm, Sxz, ps[4]);
         v[5] = fma2(dm, Syz, ps[5]);
@@ -608,15 +645,16 @@ constexpr int kVsyz = kPW * kTY, kVszz = kVsyz + kTX * kPH, kVA = kVszz + kTX * 
 constexpr int kVsyy = kPW * kPH, kVsxx = kVsyy + kTX * kPH, kVB = kVsxx + kPW * kTY;
 using VelFlow = Flow<kVA, kVB, kDepth>;
 
-// MODE kFwd: gridext with its absorbing layers; kBwd: gridphy with the rim
-// orders, backwards in time.
+// MODE kFwd, kRev: gridext with its absorbing layers; kBwd: gridphy with the
+// rim orders, backwards in time.  Of the three differences of a velocity, kFwd
+// rounds the x term and joins y, then z; the others round y and join x, then z.
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, 2)
     vel_tile(GridDev g, const __grid_constant__ VelMaps maps, const __grid_constant__ WaveDev w,
              const float *__restrict__ bdt, const float *__restrict__ vpm, float dt, int rec_w,
              const __grid_constant__ TileGeo q, int *err) {
     using FL = VelFlow;
-    constexpr bool kCp = MODE != kBwd;
+    constexpr bool kCp = MODE != kBwd, kXFirst = MODE == kFwd;
     extern __shared__ __align__(128) float sm[];
     __shared__ __align__(8) uint64_t bars[FL::SA + FL::D];
     __shared__ f2 rows[5][4];
@@ -659,7 +697,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         const int a = (tid & 31) >> 1;
         if (a < 4) pf = (a == 0 ? bdt : w.f[VX + a - 1]) + t.line(g, q) + kAhead * sz;
     }
-    const f2 rdx = dup(1.0f / g.dx), rdy = dup(1.0f / g.dy), rdz = dup(1.0f / g.dz), dt2 = dup(dt);
+    const f2 rdx = dup(1.0f / g.dx), rdy = dup(1.0f / g.dy), dt2 = dup(dt);
     const bool ph0 = t.x >= m && t.x < m + g.px, ph1 = t.x + 1 >= m && t.x + 1 < m + g.px;
     const bool yph = t.y >= m && t.y < m + g.py;
     const bool xab = kCp && ((t.mask & 1 && !ph0) || (t.mask & 2 && !ph1)), yab = kCp && live && !yph;
@@ -669,7 +707,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         copy_commit();
     }
     int zclass = -1;
-    f2 cx[4];
+    f2 cx[5];
     if (!kCp) {
         const int o0 = rim_order(min(max(t.x - m, 0), g.px - 1), g.px, rec_w);
         const int o1 = rim_order(min(max(t.x + 1 - m, 0), g.px - 1), g.px, rec_w);
@@ -698,15 +736,13 @@ __global__ void __launch_bounds__(kThreads, 2)
         if (pf && k + kAhead < t.n) prefetch_line(pf + (long long)k * sz);
         ok = rd.wait();
         if (!ok) break;
-        const bool zph = !zabs(z);
+        const bool zph = !zabs(z), p0 = ph0 && yph && zph, p1 = ph1 && yph && zph;
+        const bool ab = kCp && !(p0 && p1);  // a cell of the pair lies in a layer
         f2 vp = 0;
         if (kCp) {
             if (zclass != (int)zph) {
                 zclass = zph;
-                const bool p = yph && zph;
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    cx[j] = pk(p && ph0 ? q.taps[4][j] : q.taps[2][j], p && ph1 ? q.taps[4][j] : q.taps[2][j]);
+                set_weights(cx, p0, p1, q);
             }
             copy_wait1();
             __syncwarp();
@@ -714,39 +750,78 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
         const int ob = rd.b * kVB;
         f2 mx, my, mz, no;
-        f2 Dx = diff_x<true>(B2 + ob, cx, rdx, no);            // sxx
-        f2 Dy = diff_x<false>(B0 + ob, cx, rdx, no);           // sxy
-        f2 Dz = diff_x<false>(A0 + rd.off[0], cx, rdx, mx);    // sxz
-        if (kCp && xab)
-            absorb_x<true>(psi.at(k & 1, 1), q.psx[0], psi.ix(z), psi.tab[t.c], psi.tab[t.c + 1], vp, dt2, Dx, Dy, Dz);
-        {
-            f2 cy[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) cy[j] = kCp ? cx[j] : rows[rim_order(t.y - m, g.py, rec_w)][j];
-            f2 a = diff_y<false, kPW>(B0 + ob, cy, rdy);          // sxy
-            f2 b = diff_y<true, kTX>(B1 + ob, cy, rdy);           // syy
-            f2 c = diff_y<false, kTX>(A1 + rd.off[0], cy, rdy);   // syz
-            if (kCp && yab)
-                absorb_yz<true>(psi.at(k & 1, 4), q.psy[0], psi.iy(z), psi.tab[kTX + t.r], vp, dt2, b, a, c);
-            Dx = add2(Dx, a);
-            Dy = add2(Dy, b);
-            Dz = add2(Dz, c);
+        f2 Dx = diff_x<true, kCp>(B2 + ob, cx, no);            // sxx
+        f2 Dy = diff_x<false, kCp>(B0 + ob, cx, no);           // sxy
+        f2 Dz = diff_x<false, kCp>(A0 + rd.off[0], cx, mx);    // sxz
+        if (kXFirst) {
+            Dx = mul2(Dx, rdx);
+            Dy = mul2(Dy, rdx);
+            Dz = mul2(Dz, rdx);
         }
-        f2 cz[4];
+        if (ab) {
+            if (!kXFirst) {
+                const Join j(p0, p1, 1.0f / g.dx);
+                Dx = mul2(Dx, j.S);
+                Dy = mul2(Dy, j.S);
+                Dz = mul2(Dz, j.S);
+            }
+            if (xab)
+                absorb_x<true>(psi.at(k & 1, 1), q.psx[0], psi.ix(z), psi.tab[t.c], psi.tab[t.c + 1], vp, dt2, Dx, Dy, Dz);
+        }
+        {
+            f2 cy[5];
 #pragma unroll
-        for (int j = 0; j < 4; j++) cz[j] = kCp ? cx[j] : rows[rim_order(z - m, g.pz, rec_w)][j];
+            for (int j = 0; j < (kCp ? 5 : 4); j++) cy[j] = kCp ? cx[j] : rows[rim_order(t.y - m, g.py, rec_w)][j];
+            f2 a = diff_y<false, kCp, kPW>(B0 + ob, cy);          // sxy
+            f2 b = diff_y<true, kCp, kTX>(B1 + ob, cy);           // syy
+            f2 c = diff_y<false, kCp, kTX>(A1 + rd.off[0], cy);   // syz
+            if (!kXFirst) {
+                a = mul2(a, rdy);
+                b = mul2(b, rdy);
+                c = mul2(c, rdy);
+            }
+            f2 R = kXFirst ? rdy : rdx;
+            if (ab) {
+                const Join j(p0, p1, kXFirst ? 1.0f / g.dy : 1.0f / g.dx);
+                if (kXFirst) {
+                    a = mul2(a, j.S);
+                    b = mul2(b, j.S);
+                    c = mul2(c, j.S);
+                }
+                if (yab)
+                    absorb_yz<true>(psi.at(k & 1, 4), q.psy[0], psi.iy(z), psi.tab[kTX + t.r], vp, dt2, b, a, c);
+                R = j.R;
+            }
+            Dx = kXFirst ? fma2(a, R, Dx) : fma2(Dx, R, a);
+            Dy = kXFirst ? fma2(b, R, Dy) : fma2(Dy, R, b);
+            Dz = kXFirst ? fma2(c, R, Dz) : fma2(Dz, R, c);
+        }
+        f2 cz[5];
+#pragma unroll
+        for (int j = 0; j < (kCp ? 5 : 4); j++) cz[j] = kCp ? cx[j] : rows[rim_order(z - m, g.pz, rec_w)][j];
         my = at2(A1 + rd.off[0]);
         mz = at2(A2 + rd.off[0]);
-        f2 a = diff_z<false>(A0, rd.off, mx, wx, cz, rdz);  // sxz
-        f2 b = diff_z<false>(A1, rd.off, my, wy, cz, rdz);  // syz
-        f2 c = diff_z<true>(A2, rd.off, mz, wz, cz, rdz);   // szz
+        f2 a = diff_z<false, kCp>(A0, rd.off, mx, wx, cz);  // sxz
+        f2 b = diff_z<false, kCp>(A1, rd.off, my, wy, cz);  // syz
+        f2 c = diff_z<true, kCp>(A2, rd.off, mz, wz, cz);   // szz
         rd.release();
         rd.next(kVA);
-        if (kCp && live && !zph)
-            absorb_yz<true>(psi.at(k & 1, 7), q.psz[0], psi.iz(g, z), psi.zrow(k & 1), vp, dt2, c, a, b);
+        f2 R = dup(1.0f / g.dz);
+        if (ab) {
+            const Join j(p0, p1, 1.0f / g.dz);
+            a = mul2(a, j.S);
+            b = mul2(b, j.S);
+            c = mul2(c, j.S);
+            if (live && !zph)
+                absorb_yz<true>(psi.at(k & 1, 7), q.psz[0], psi.iz(g, z), psi.zrow(k & 1), vp, dt2, c, a, b);
+            R = j.R;
+        }
+        Dx = fma2(a, R, Dx);
+        Dy = fma2(b, R, Dy);
+        Dz = fma2(c, R, Dz);
         // the stored dt / rho is of the forward step
         const f2 b1 = MODE == kBwd ? mul2(pb, pk(-1.f, -1.f)) : pb;
-        const f2 v[3] = {fma2(b1, add2(Dx, a), pv[0]), fma2(b1, add2(Dy, b), pv[1]), fma2(b1, add2(Dz, c), pv[2])};
+        const f2 v[3] = {fma2(b1, Dx, pv[0]), fma2(b1, Dy, pv[1]), fma2(b1, Dz, pv[2])};
         float *const dst[3] = {w.f[VX], w.f[VY], w.f[VZ]};
         put2(dst, v, o, t.mask);
         // the first warp refills what every live warp has given back
@@ -767,7 +842,7 @@ struct PvelMaps {
 template <bool FB, bool RP>
 using PvelFlow = Flow<((FB ? 1 : 0) + (RP ? 1 : 0)) * kSField, 0, kDepth>;
 
-__device__ __forceinline__ f2 dot3(const f2 *a, const f2 *b) { return fma2(a[2], b[2], fma2(a[1], b[1], mul2(a[0], b[0]))); }
+__device__ __forceinline__ f2 dot3(const f2 *a, const f2 *b) { return fma2(a[2], b[2], fma2(a[0], b[0], mul2(a[1], b[1]))); }
 
 // The P-wave velocities over gridphy, from the pressure-like field sau (Dp on
 // every axis): with RP the receiver wavefield's, forwards in time; with FB
@@ -858,21 +933,21 @@ __global__ void __launch_bounds__(kThreads, 2)
         const float *F = S + rd.off[0];
         f2 mid, d[3], e[3], c[4];
         if (FB) {
-            d[0] = diff_x<true>(F, cx, rdx, mid);
+            d[0] = mul2(diff_x<true, false>(F, cx, mid), rdx);
 #pragma unroll
             for (int j = 0; j < 4; j++) c[j] = rows[rim_order(t.y - m, g.py, rec_w)][j];
-            d[1] = diff_y<true, kPW>(F, c, rdy);
+            d[1] = mul2(diff_y<true, false, kPW>(F, c), rdy);
 #pragma unroll
             for (int j = 0; j < 4; j++) c[j] = rows[rim_order(z - m, g.pz, rec_w)][j];
-            d[2] = diff_z<true>(S, rd.off, mid, wf, c, rdz);
+            d[2] = mul2(diff_z<true, false>(S, rd.off, mid, wf, c), rdz);
         }
         if (RP) {
             constexpr int R = FB ? kSField : 0;
 #pragma unroll
             for (int j = 0; j < 4; j++) c[j] = rows[kPhyHalf][j];
-            e[0] = diff_x<true>(F + R, c, rdx, mid);
-            e[1] = diff_y<true, kPW>(F + R, c, rdy);
-            e[2] = diff_z<true>(S + R, rd.off, mid, wr, c, rdz);
+            e[0] = mul2(diff_x<true, false>(F + R, c, mid), rdx);
+            e[1] = mul2(diff_y<true, false, kPW>(F + R, c), rdy);
+            e[2] = mul2(diff_z<true, false>(S + R, rd.off, mid, wr, c), rdz);
         }
         rd.release();
         rd.next(AF);
@@ -1067,6 +1142,7 @@ int k_make_tile_maps(const GridDev &g, const WaveDev &w, bool phy, float4 *const
                                                    {(const void *)stress_tile<kRev>, stress_smem<kRev>()},
                                                    {(const void *)stress_tile<kBwd>, stress_smem<kBwd>()},
                                                    {(const void *)vel_tile<kFwd>, vel_smem<kFwd>()},
+                                                   {(const void *)vel_tile<kRev>, vel_smem<kRev>()},
                                                    {(const void *)vel_tile<kBwd>, vel_smem<kBwd>()},
                                                    {(const void *)pvel_tile<true, true>, pvel_smem<true, true>()},
                                                    {(const void *)pvel_tile<true, false>, pvel_smem<true, false>()},
@@ -1112,10 +1188,15 @@ int k_vel_tile(int mode, const GridDev &g, const WaveDev &w, const float *bdt, c
     std::memcpy(&vm, m.v, sizeof(vm));
     const int grid = m.geo.ntx * m.geo.nty * m.geo.Q;
     cudaStream_t s = (cudaStream_t)stream;
-    if (mode == kBwd)
-        vel_tile<kBwd><<<grid, kThreads, vel_smem<kBwd>(), s>>>(g, vm, w, bdt, vp, dt, rec_w, m.geo, m.err);
-    else
-        vel_tile<kFwd><<<grid, kThreads, vel_smem<kFwd>(), s>>>(g, vm, w, bdt, vp, dt, rec_w, m.geo, m.err);
+#define JV_VT(M) vel_tile<M><<<grid, kThreads, vel_smem<M>(), s>>>(g, vm, w, bdt, vp, dt, rec_w, m.geo, m.err)
+    switch (mode) {
+    case kFwd:
+    case kRtmFwd: JV_VT(kFwd); break;
+    case kRev: JV_VT(kRev); break;
+    case kBwd: JV_VT(kBwd); break;
+    default: return (int)cudaErrorInvalidValue;
+    }
+#undef JV_VT
     return (int)cudaGetLastError();
 }
 

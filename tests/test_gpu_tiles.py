@@ -67,6 +67,123 @@ def test_tile_kernels_unequal_spacing(oracle, synth, dx, dy, dz):
         assert rel_l2(a, b) <= 2e-5, rel_l2(a, b)
 
 
+# ------------------------------------------------ rounding, bit for bit
+
+F32 = np.float32
+
+
+def _fma(a, b, c):
+    """a b + c in FP32 with one rounding: the exact product, its sum with c rounded to odd in FP64, then to FP32."""
+    p = np.asarray(a, F32).astype(np.float64) * np.asarray(b, F32).astype(np.float64)
+    p, c = np.broadcast_arrays(p, np.asarray(c, F32).astype(np.float64))
+    s = p + c
+    t = s - p
+    err = (p - (s - t)) + (c - t)
+    bits = s.view(np.int64)
+    step = np.where((err != 0) & (bits & 1 == 0), np.where((err > 0) == (s > 0), 1, -1), 0)
+    return (bits + step).view(np.float64).astype(F32)
+
+
+class _Interior:
+    """One FP32 wavefield of a grid so large that nothing reaches its faces; arrays (z, y, x), axis 0 is x."""
+    TAPS = [F32(c) for c in (1225 / 1024, -245 / 3072, 49 / 5120, -5 / 7168)]
+    SUMS = (("vx", (("sxx", 0, True), ("sxy", 1, False), ("sxz", 2, False))),
+            ("vy", (("sxy", 0, False), ("syy", 1, True), ("syz", 2, False))),
+            ("vz", (("sxz", 0, False), ("syz", 1, False), ("szz", 2, True))))
+
+    def __init__(self, s):
+        vp, vs, rho = (np.asarray(a, F32) for a in (s.vp, s.vs, s.rho))
+        self.dt, self.rd, self.bdt = F32(s.dt), [F32(1) / F32(d) for d in (s.dx, s.dy, s.dz)], F32(s.dt) / rho
+        vs2 = vs * vs
+        self.lam, self.mu = rho * (vp * vp - F32(2) * vs2), rho * vs2
+        self.f = {k: np.zeros_like(vp) for k in ("vx", "vy", "vz", "sxx", "syy", "szz", "sxy", "sxz", "syz", "sau",
+                                                 "px", "py", "pz")}
+
+    def diff(self, k, axis, plus):
+        def at(n):
+            return np.roll(self.f[k], -n, 2 - axis)
+        d = [at(q + 1) - at(-q) if plus else at(q) - at(-q - 1) for q in range(4)]
+        t = self.TAPS[0] * d[0]
+        for q in (1, 2, 3):
+            t = _fma(self.TAPS[q], d[q], t)
+        return t
+
+    def velocity(self, forward, sign=1):
+        rx, ry, rz = self.rd
+        for v, terms in self.SUMS:
+            x, y, z = (self.diff(*t) for t in terms)
+            d = _fma(y, ry, x * rx) if forward else _fma(x, rx, y * ry)
+            self.f[v] = _fma(F32(sign) * self.bdt, _fma(z, rz, d), self.f[v])
+
+    def p_velocity(self, sign):
+        for axis, p in enumerate(("px", "py", "pz")):
+            self.f[p] = _fma(F32(sign) * self.bdt, self.diff("sau", axis, True) * self.rd[axis], self.f[p])
+
+    def stress(self, sign=1, source=None, value=0):
+        f, dt, (rx, ry, rz) = self.f, F32(sign) * self.dt, self.rd
+        if source is not None:
+            for k in ("sxx", "syy", "szz"):
+                f[k][source] = f[k][source] + F32(sign) * value
+        nx, ny, nz = (self.diff(k, a, False) * self.rd[a] for a, k in enumerate(("vx", "vy", "vz")))
+        lam, mu = self.lam, self.mu
+        l2m = _fma(mu, F32(2), lam)
+        new = {"sxx": _fma(dt, _fma(lam, nz, _fma(l2m, nx, lam * ny)), f["sxx"]),
+               "syy": _fma(dt, _fma(lam, nz, _fma(lam, nx, l2m * ny)), f["syy"]),
+               "szz": _fma(dt, _fma(l2m, nz, _fma(lam, nx, lam * ny)), f["szz"]),
+               "sau": _fma(dt * l2m, (nx + ny) + nz, f["sau"])}
+        for k, (a, i, r), (b, j, q) in (("sxy", ("vy", 0, rx), ("vx", 1, ry)), ("sxz", ("vz", 0, rx), ("vx", 2, rz)),
+                                        ("syz", ("vz", 1, ry), ("vy", 2, rz))):
+            new[k] = _fma(dt * mu, _fma(self.diff(a, i, True), r, self.diff(b, j, True) * q), f[k])
+        f.update(new)
+
+
+def _wavelet(s):
+    n0 = int(np.floor(F32(1.3) / F32(s.fm) / F32(s.dt) + F32(0.5)))
+    a2 = [(np.pi * float(F32(s.fm)) * float(F32(i - n0) * F32(s.dt))) ** 2 for i in range(s.nt)]
+    return [F32(1e4 * (1 - 2 * x) * np.exp(-x)) for x in a2]
+
+
+@pytest.mark.parametrize("n,dx,dy,dz", [((57, 58, 60), 10.0, 10.0, 10.0), ((64, 56, 58), 10.0, 12.5, 8.0)])
+def test_sums_of_differences_round_once(synth, n, dx, dy, dz):
+    """Three steps of modelling and of migration from the middle of a grid, where no layer is reached: every trace
+    and image equals its FP32 sums with the stated fused multiply-adds, bit for bit (no tolerance)."""
+    c = tuple(k // 2 for k in n)
+    s = synth.small_case(n=n, pml=4, nt=3, seed=81, dx=dx, fm=300.0, dt=2e-4, shot_idx=[c])
+    recs = np.array([(c[0] + i, c[1] + j, c[2] + k) for i in range(-9, 10, 3) for j in (-7, 0, 2) for k in (-5, 1)])
+    s.dy, s.dz = dy, dz
+    s.shots = (np.array([c]) * np.array([dx, dy, dz])).astype(F32)
+    s.recvs = (recs * np.array([dx, dy, dz])).astype(F32)
+    obs = [(1e-3 * np.random.default_rng(q).standard_normal((len(recs), s.nt))).astype(F32) for q in range(3)]
+    with jv.Context.from_survey(s) as ctx:
+        tr = ctx.forward(0)
+        ctx.rtm_shot(0, obs)
+        raw = ctx.images()
+    w, src, at = _Interior(s), c[::-1], tuple(recs.T[::-1])
+    wavelet, V, P = _wavelet(s), ("vx", "vy", "vz"), ("px", "py", "pz")
+    for it in range(s.nt):
+        w.velocity(True)
+        w.stress(1, src, wavelet[it])
+        for q, v in enumerate(V):
+            assert np.array_equal(tr[q][:, it], w.f[v][at]), (it, v)
+    r = _Interior(s)
+    img = {k: np.zeros_like(w.lam) for k in ("ip", "pp", "ps", "sp", "ss")}
+    for it in range(s.nt - 1, -1, -1):
+        for q, v in enumerate(V):
+            r.f[v][at] += obs[q][:, it]
+        w.stress(-1, src, wavelet[it])
+        w.velocity(False, -1)
+        r.velocity(False)
+        w.p_velocity(-1)
+        r.p_velocity(1)
+        sp, rp = [w.f[k] for k in P], [r.f[k] for k in P]
+        ss, rs = ([u.f[v] - p for v, p in zip(V, pp)] for u, pp in ((w, sp), (r, rp)))
+        for k, a, b in (("ip", sp, sp), ("pp", sp, rp), ("ps", sp, rs), ("sp", ss, rp), ("ss", ss, rs)):
+            img[k] = img[k] + _fma(a[2], b[2], _fma(a[0], b[0], a[1] * b[1]))
+        r.stress()
+    for k in img:
+        assert np.abs(img[k]).max() > 0 and np.array_equal(raw[k].astype(F32), img[k]), k
+
+
 def test_tile_layout_covers_every_cell():
     """The columns of every grid fall in exactly one tile, start pairs on
     8-byte boundaries, and the memory variables of a pair lie within their
