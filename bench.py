@@ -229,6 +229,17 @@ def kernel_bytes(s, name):
     return None
 
 
+def kernel_rows(prof, s, att, peak):
+    """Lines of the kernel table, the longest first; an entry without launches has no rate."""
+    tot = sum(ms for ms, _ in prof.values())
+    for k, (ms, n) in sorted(prof.items(), key=lambda kv: -kv[1][0]):
+        b, us, nan = kernel_bytes(s, k), 1000.0 * ms / max(n, 1), float("nan")
+        gbs = b / (us * 1e-6) / 1e9 if b and us > 0 else nan
+        a = att.get(FOOTPRINT.get(k))
+        yield (f"  {k:22s} {n:8d} {us:10.1f} {ms / tot if tot > 0 else nan:7.1%} {b or 0:12.4g} {gbs:8.0f} "
+               f"{gbs / peak:8.1%} {gbs / a if a else nan:14.1%}")
+
+
 def cpu_sample(s, oracle, seconds_target=20.0, max_steps=200):
     """FP64 oracle on all host cores: a bounded sample of one RTM shot."""
     p = oracle.Problem(s.nx, s.ny, s.nz, s.pml, s.dx, s.dy, s.dz, s.dt, s.fm, s.T, s.rec_width, s.shots,
@@ -835,13 +846,8 @@ def main():
                   file=sys.stderr)
             print(f"  {'kernel':22s} {'launches':>8s} {'us/launch':>10s} {'share':>7s} {'alg. bytes':>12s} "
                   f"{'GB/s':>8s} {'of peak':>8s} {'of attainable':>14s}", file=sys.stderr)
-            for k, (kms, kn) in sorted(prof.items(), key=lambda kv: -kv[1][0]):
-                kb = kernel_bytes(s, k)
-                us = 1000.0 * kms / max(kn, 1)
-                gbs = kb / (us * 1e-6) / 1e9 if kb else float("nan")
-                a = att.get(FOOTPRINT.get(k))
-                print(f"  {k:22s} {kn:8d} {us:10.1f} {kms / tot:7.1%} {kb or 0:12.4g} {gbs:8.0f} "
-                      f"{gbs / peak:8.1%} {(gbs / a) if a else float('nan'):14.1%}", file=sys.stderr)
+            for row in kernel_rows(prof, s, att, peak):
+                print(row, file=sys.stderr)
             print("  attainable: " + ", ".join(f"{r} read + {w} written {g:.0f} GB/s" for (r, w), g in att.items()),
                   file=sys.stderr)
         if b is not None and n > 0:

@@ -71,6 +71,7 @@ const Shape kShapes[] = {
     {10, 3, launch<10, 3>},   // velocity update, no P-wave velocities
     {12, 7, launch<12, 7>},   // stress update with sau
     {14, 6, launch<14, 6>},   // velocity update with P-wave velocities
+    {20, 11, launch<20, 11>}, // P-wave velocities of both wavefields with imaging
     {25, 11, launch<25, 11>}, // backward velocity update with imaging
 };
 
@@ -87,7 +88,7 @@ extern "C" jv_status jv_stream_probe(int device, int n_read, int n_write, size_t
     for (const Shape &s : kShapes)
         if (s.nr == n_read && s.nw == n_write) sh = &s;
     if (!sh)
-        return fail(JV_EINVAL, "jv_stream_probe: (reads, writes) must be one of (1,1) (2,1) (10,3) (12,7) (14,6) (25,11)");
+        return fail(JV_EINVAL, "jv_stream_probe: (reads, writes) must be one of (1,1) (2,1) (10,3) (12,7) (14,6) (20,11) (25,11)");
     if (cudaSetDevice(device) != cudaSuccess) return fail(JV_ECUDA, "jv_stream_probe: no such device");
     const int na = n_read + n_write;
     std::vector<float *> bufs(na, nullptr);

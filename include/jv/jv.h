@@ -491,7 +491,8 @@ jv_status jv_forward_noalloc(const jv_grid *grid, const float *d_vp, const float
  * array per thread, every load issued before the stores), in GB/s of bytes
  * moved, from the median device time of `reps` launches after one warm-up.
  * The supported (n_read, n_write) pairs are the footprints of this
- * library's kernels and a copy: (1,1) (2,1) (10,3) (12,7) (14,6) (25,11).
+ * library's kernels and a copy: (1,1) (2,1) (10,3) (12,7) (14,6) (20,11)
+ * (25,11).
  * Allocates its arrays on `device` and frees them before it returns.  A
  * diagnostic for the roofline of many-array kernels; no counterpart in the
  * reference. */

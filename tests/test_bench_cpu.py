@@ -2,6 +2,7 @@
 rule, and the algorithmic byte model the roofline divides by."""
 import json
 import os
+import re
 import subprocess
 import sys
 
@@ -10,6 +11,7 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path.insert(0, ROOT)
 import bench  # noqa: E402
+from conftest import pkg  # noqa: E402
 
 
 def _run(*args, env=None):
@@ -61,6 +63,23 @@ def test_byte_model(synth, n, pml):
     assert bench.kernel_bytes(s, "stress_fz_rev") == (bench.kernel_bytes(s, "stress_phy_rev")
                                                       + bench.kernel_bytes(s, "stress_pml_sau"))
     assert bench.kernel_bytes(s, "vowr_pack") is None
+
+
+def test_every_footprint_has_a_bandwidth_probe():
+    jv = pkg()
+    with pytest.raises(jv.JvError) as e:  # names the pairs it takes; refused before a device is looked for
+        jv.stream_probe(99, 99, 4)
+    pairs = {tuple(map(int, p)) for p in re.findall(r"\((\d+),(\d+)\)", str(e.value))}
+    assert len(pairs) >= 6 and set(bench.FOOTPRINT.values()) <= pairs, set(bench.FOOTPRINT.values()) - pairs
+
+
+def test_kernel_table_takes_entries_without_launches(synth):
+    s = synth.scaled_cfg2(44, 10, pml=10)
+    prof = {k: (1.5, 3) for k in bench.FOOTPRINT}
+    prof.update({"vel_pml": (0.0, 0), "vel_phy_rev": (0.0, 0), "record": (0.2, 3)})
+    rows = list(bench.kernel_rows(prof, s, {v: 4000.0 for v in bench.FOOTPRINT.values()}, 6459.6))
+    assert len(rows) == len(prof) and "nan" in next(r for r in rows if "vel_pml" in r)
+    assert all(len(list(bench.kernel_rows({"vel_pml": z}, s, {}, 1.0))) == 1 for z in ((0.0, 0), (0.0, 2)))
 
 
 def test_traffic_read_from_the_committed_profile():

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 jv = pkg()
 
 
-@pytest.mark.parametrize("nr,nw", [(1, 1), (2, 1), (10, 3), (12, 7), (14, 6), (25, 11)])
+@pytest.mark.parametrize("nr,nw", [(1, 1), (2, 1), (10, 3), (12, 7), (14, 6), (20, 11), (25, 11)])
 def test_stream_probe_rates(nr, nw):
     gbs = jv.stream_probe(nr, nw, 1 << 25, reps=3)  # 128 MiB per array
     assert 500.0 < gbs < 9000.0, gbs
