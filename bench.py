@@ -157,10 +157,10 @@ BYTES_PER_CELL = {
 # can move; the full-gridext kernels add CPML memory variables at the rim
 FOOTPRINT = {
     "vel_phy_bwd_image": (25, 11), "vel_phy_rev": (14, 6), "vel_phy_rtmfwd": (10, 3), "vel_phy_fwd": (10, 3),
-    "vel_fz_rtmfwd": (10, 3), "vel_fz_fwd": (10, 3), "vel_tile_rtmfwd": (10, 3), "vel_tile_fwd": (10, 3),
+    "vel_tile_rtmfwd": (10, 3), "vel_tile_fwd": (10, 3),
     "vel_tile_rev": (10, 3), "vel_tile_bwd": (10, 3), "pvel_image": (20, 11), "stress_tile_bwd": (12, 7),
     "stress_phy_bwd": (12, 7), "stress_phy_rev": (12, 7), "stress_phy_rtmfwd": (12, 7),
-    "stress_fz_rev": (12, 7), "stress_fz_rtmfwd": (12, 7),
+    "stress_tile_rev": (12, 7), "stress_tile_rtmfwd": (12, 7),
 }
 
 
@@ -208,12 +208,11 @@ def pml_bytes(s, name):
     return float(cells * per + axes * 3 * 8)
 
 
-# the full-gridext kernels (variant 4) do the work of two launches
-FUSED = {"stress_fz_fwd": ("stress_phy_fwd", "stress_pml"),
-         "stress_fz_rtmfwd": ("stress_phy_rtmfwd", "stress_pml_sau"),
-         "stress_fz_rev": ("stress_phy_rev", "stress_pml_sau"),
-         "vel_fz_fwd": ("vel_phy_fwd", "vel_pml"),
-         "vel_fz_rtmfwd": ("vel_phy_rtmfwd", "vel_pml"),
+# the tile kernels over gridext (variant 4) do the work of two of the split kernels; the receiver side's velocity
+# update leaves its P-wave velocities to pvel_image
+FUSED = {"stress_tile_fwd": ("stress_phy_fwd", "stress_pml"),
+         "stress_tile_rtmfwd": ("stress_phy_rtmfwd", "stress_pml_sau"),
+         "stress_tile_rev": ("stress_phy_rev", "stress_pml_sau"),
          "vel_tile_fwd": ("vel_phy_fwd", "vel_pml"),
          "vel_tile_rtmfwd": ("vel_phy_rtmfwd", "vel_pml"),
          "vel_tile_rev": ("vel_phy_fwd", "vel_pml")}

@@ -576,7 +576,6 @@ Status Engine::alloc_all(const float *vp, const float *vs, const float *rho) {
         tpsiF_ = (float *)p;
         JV_TRY(make_tiles());
         tiles_ = tileF_.ok;
-        wide_ = g_.nx - 4 + 10 > 256;
     }
     // the slab layout's memory variables: the other variants, tried by the
     // measured choice
@@ -889,10 +888,9 @@ Status Engine::launch_step(int kind, int off, bool advance, bool first, bool las
     switch (kind) {
     case kStepModel:
         if (tiles_) {
-            if (wide_) folded("vel_pml"), folded("vel_phy_fwd");
-            JV_L(wide_ ? "vel_tile_fwd" : "vel_fz_fwd", k_vel_tile(kFwd, g_, F_, bdt_, vp_, dt, rw, tileF_, s));
+            JV_L("vel_tile_fwd", k_vel_tile(kFwd, g_, F_, bdt_, vp_, dt, rw, tileF_, s));
             JV_TRY(order(0, stream_, side));
-            JV_L("stress_fz_fwd",
+            JV_L("stress_tile_fwd",
                  k_stress_tile(kFwd, g_, F_, lam_, mu_, vp_, dt, rw, wavelet_, st_, off, tileF_, s));
             JV_L("record", k_record(F_, rec_d_, nrec_, nt_, st_, off, s2));
             JV_TRY(order(1, side, stream_));
@@ -908,13 +906,12 @@ Status Engine::launch_step(int kind, int off, bool advance, bool first, bool las
         break;
     case kStepRtmFwd:
         if (tiles_) {
-            if (wide_) folded("vel_pml"), folded("vel_phy_rtmfwd");
-            JV_L(wide_ ? "vel_tile_rtmfwd" : "vel_fz_rtmfwd", k_vel_tile(kRtmFwd, g_, F_, bdt_, vp_, dt, rw, tileF_, s));
+            JV_L("vel_tile_rtmfwd", k_vel_tile(kRtmFwd, g_, F_, bdt_, vp_, dt, rw, tileF_, s));
             // the boundary boxes lie in the absorbing layers: packed after their update
             JV_TRY(order(0, stream_, side));
             if (!first) JV_TRY(order(2, side, stream_));  // the step before's stress boxes are packed
             JV_L("vowr_pack", k_vowr(g_, F_, vowr_, st_, off, 1, 1, s2));
-            JV_L("stress_fz_rtmfwd",
+            JV_L("stress_tile_rtmfwd",
                  k_stress_tile(kRtmFwd, g_, F_, lam_, mu_, vp_, dt, rw, wavelet_, st_, off, tileF_, s));
             JV_TRY(order(1, side, stream_));
             JV_TRY(order(0, stream_, side));
@@ -946,12 +943,12 @@ Status Engine::launch_step(int kind, int off, bool advance, bool first, bool las
             // the receiver side's velocities, absorbing layers included; its
             // P-wave velocities follow in the imaging kernel
             JV_L("inject_rec", k_inject_rec(R_, rec_d_, nrec_, nt_, st_, off, s));
-            folded("vel_pml"), folded("vel_phy_rev");
             JV_L("vel_tile_rev", k_vel_tile(kRev, g_, R_, bdt_, vp_, dt, rw, tileR_, s));
             JV_TRY(order(1, side, stream_));
             JV_L("pvel_image", k_pvel_tile(g_, &F_, &tileFB_, R_, tileRB_, true, bdt_, rw, &shot_img_, s));
             if (!last) JV_TRY(order(0, stream_, side));
-            JV_L("stress_fz_rev", k_stress_tile(kRev, g_, R_, lam_, mu_, vp_, dt, rw, wavelet_, st_, off, tileR_, s));
+            JV_L("stress_tile_rev",
+                 k_stress_tile(kRev, g_, R_, lam_, mu_, vp_, dt, rw, wavelet_, st_, off, tileR_, s));
         } else {
             JV_L("inject_rec", k_inject_rec(R_, rec_d_, nrec_, nt_, st_, off, s));
             JV_L("stress_phy_bwd",

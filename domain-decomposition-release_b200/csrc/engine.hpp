@@ -188,7 +188,6 @@ class Engine {
 
   private:
     bool tiles_ = false;          // the time loops run variant 4's tile kernels
-    bool wide_ = false;           // a gridext row is wider than one 256-float box
     int *zm_err_ = nullptr;       // device flag of variant 3's bounded waits
     Status check_zm_err();
     size_t field_elems_ = 0;  // elements per pitched field
@@ -241,10 +240,6 @@ class Engine {
     std::vector<cudaEvent_t> prof_pool_;
     size_t prof_used_ = 0;
     int prof_id(const char *name);
-    // a phase that another phase's kernel carries: listed with no launches
-    void folded(const char *name) {
-        if (prof_) prof_id(name);
-    }
     cudaEvent_t prof_event();
     Status prof_collect();
 

@@ -97,10 +97,9 @@ typedef struct jv_options {
     int pml_min_blocks; /* absorbing-layer kernels: the same (0 -> 4)            */
     int planes_per_thread;     /* variant 2: z planes a thread updates, 1 or 2 (0 -> 1) */
     int pml_planes_per_thread; /* absorbing-layer kernels: the same (0 -> 1)      */
-    int run_chunks;     /* variant 4: chunks each tile's planes are cut into for the
-                           persistent kernels' run schedule (0 -> the cost model's
-                           choice; with kernel_variant -1 the measured choice among the
-                           cost model's three best); jv_get_kernel_config reports it */
+    int run_chunks;     /* variant 4: chunks each tile's planes are cut into (0 -> the cost
+                           model's choice; with kernel_variant -1 the measured choice among
+                           the cost model's three best); jv_get_kernel_config reports it */
     int autotune;       /* 1 (default): at creation, time the knobs that cannot change a result --
                            variant 4's run chunking among the cost model's three best and the
                            float4 kernels' block shape -- on this grid and keep the fastest, per
@@ -456,9 +455,7 @@ jv_status jv_rtm_reverse_end(jv_ctx *c);
  * directly (no graphs) and bracket each launch with CUDA events on the
  * context's stream; jv_profile_entry returns, for entry idx, the kernel
  * name, the summed device time and the launch count since profiling was
- * switched on (JV_EINVAL past the last entry).  A phase that another
- * phase's kernel carries (an absorbing layer's update within gridext's) is
- * listed with no launches.  The reference prints
+ * switched on (JV_EINVAL past the last entry).  The reference prints
  * per-shot times only (cuda_tic/cuda_toc, .jarvis_0_meta/.jarvis_0_math/
  * jarvis_2_device_math_bones.hpp:26-38). */
 jv_status jv_set_profiling(jv_ctx *c, int on);

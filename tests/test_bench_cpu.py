@@ -59,9 +59,9 @@ def test_byte_model(synth, n, pml):
     shell = (N - 4) ** 3 - n ** 3
     vp = bench.kernel_bytes(s, "vel_pml")
     assert 56 * shell + 24 * shell <= vp <= 56 * shell + 3 * 24 * shell
-    # a full-gridext kernel does the work of its interior and absorbing-layer pair
-    assert bench.kernel_bytes(s, "stress_fz_rev") == (bench.kernel_bytes(s, "stress_phy_rev")
-                                                      + bench.kernel_bytes(s, "stress_pml_sau"))
+    # a tile kernel over gridext does the work of an interior and absorbing-layer pair
+    assert bench.kernel_bytes(s, "stress_tile_rev") == (bench.kernel_bytes(s, "stress_phy_rev")
+                                                        + bench.kernel_bytes(s, "stress_pml_sau"))
     assert bench.kernel_bytes(s, "vowr_pack") is None
 
 

@@ -34,8 +34,8 @@ SMALL = [
 ]
 
 
-# interior kernels: one plane per block, z-marching, x-vectorised, + TMA z-marching stress, + the stress update
-# of the absorbing layers in the same TMA kernel (variant 4; even pml_num and nx, else variant 3's kernels)
+# stencil kernels: one plane per block, z-marching, x-vectorised, + TMA z-marching stress, z-marching tiles that
+# carry the absorbing layers (variant 4)
 VARIANTS = [0, 1, 2, 3, 4]
 
 
@@ -204,9 +204,8 @@ def test_launch_options_do_not_change_results(synth, kw):
         assert rel_l2(i0[k], i1[k]) <= 2e-5, k
 
 
-# grids on which variant 4's full-gridext stress and velocity kernels run (even pml_num and
-# nx): region boundaries at every tile-row offset, the smallest pml, sources
-# and receivers next to the absorbing layers
+# variant 4's kernels, gridphy and absorbing layers in one: region boundaries at many tile-row offsets, the smallest
+# pml, sources and receivers next to the absorbing layers
 FULL = [
     dict(n=(26, 14, 16), pml=8, nt=120, seed=31, shot_idx=[(1, 2, 1)]),
     dict(n=(40, 12, 10), pml=10, nt=110, seed=32, nrec=40),
@@ -216,7 +215,15 @@ FULL = [
 
 
 def _kernels(ctx):
-    return set(ctx.profile())
+    p = ctx.profile()
+    assert all(n > 0 for _, n in p.values()), p
+    return set(p)
+
+
+# what variant 4 launches: nothing but the tile kernels and the small ones
+TILE_FORWARD = {"vel_tile_fwd", "stress_tile_fwd", "record", "step_advance"}
+TILE_RTM = {"vel_tile_rtmfwd", "vowr_pack", "stress_tile_rtmfwd", "stress_tile_bwd", "vowr_unpack", "vel_tile_bwd",
+            "inject_rec", "vel_tile_rev", "pvel_image", "stress_tile_rev", "step_advance"}
 
 
 @pytest.mark.parametrize("kw", FULL)
@@ -228,7 +235,7 @@ def test_full_stress_kernel_forward_vs_oracle(oracle, synth, kw):
         ctx.set_profiling(True)
         ctx.forward(0)
         names = _kernels(ctx)
-    assert {"stress_fz_fwd", "vel_fz_fwd"} <= names and not {"stress_pml", "vel_pml"} & names, names
+    assert names == TILE_FORWARD, names
     for a, b in zip(tr, ref):
         assert np.all(np.isfinite(a))
         assert rel_l2(a, b) <= 2e-5, rel_l2(a, b)
@@ -247,9 +254,7 @@ def test_full_stress_kernel_rtm_vs_oracle(oracle, synth, kw, w):
         ctx.rtm_shot(0, obs32)
         names = _kernels(ctx)
         raw = ctx.images()
-    # the receiver side's velocity update keeps the split kernels
-    assert {"stress_fz_rtmfwd", "stress_fz_rev", "vel_fz_rtmfwd", "vel_pml", "vel_phy_rev"} <= names, names
-    assert "stress_pml_sau" not in names, names
+    assert names == TILE_RTM, names
     for k in ("ip", "pp", "ps", "sp", "ss"):
         assert np.all(np.isfinite(raw[k]))
         assert rel_l2(raw[k], ref[k]) <= 5e-5, (w, k, rel_l2(raw[k], ref[k]))
@@ -304,8 +309,7 @@ def test_16bit_boundary_store_vs_oracle(oracle, synth, prec, img_tol, w):
         assert np.isfinite(e) and e <= img_tol, (k, err)
 
 
-# grids wide enough that variant 4 cuts the x range into tiles (2-3 x tiles;
-# the absorbing strips ride with the first and last tile)
+# rows of many 32-column tiles, wider than the 256 floats of a TMA box
 WIDE = [
     dict(n=(260, 10, 12), pml=8, nt=90, seed=51, shot_idx=[(3, 5, 6)], nrec=30),
     dict(n=(300, 9, 10), pml=10, nt=80, seed=52, shot_idx=[(296, 4, 5)]),
@@ -321,8 +325,7 @@ def test_full_kernels_x_tiles_forward_vs_oracle(oracle, synth, kw):
         ctx.set_profiling(True)
         tr = ctx.forward(0)
         names = _kernels(ctx)
-    # x-tiled grids: fused stress update, split velocity update
-    assert {"stress_fz_fwd", "vel_pml", "vel_phy_fwd"} <= names and "vel_fz_fwd" not in names, names
+    assert names == TILE_FORWARD, names
     for a, b in zip(tr, ref):
         assert np.all(np.isfinite(a))
         assert rel_l2(a, b) <= 2e-5, rel_l2(a, b)
@@ -367,7 +370,7 @@ def test_full_kernels_x_tiles_rtm_vs_oracle(oracle, synth):
         ctx.rtm_shot(0, [o.astype(np.float32) for o in obs])
         names = _kernels(ctx)
         raw = ctx.images()
-    assert {"stress_fz_rtmfwd", "stress_fz_rev"} <= names and "stress_pml_sau" not in names, names
+    assert names == TILE_RTM, names
     for k in ("ip", "pp", "ps", "sp", "ss"):
         assert rel_l2(raw[k], ref[k]) <= 5e-5, (k, rel_l2(raw[k], ref[k]))
 
@@ -416,10 +419,9 @@ def test_measured_kernel_choice(oracle, synth):
 
 
 def test_tile_with_a_mixed_warp(oracle, synth):
-    """A grid whose x tiles fit one CTA only without rounding the physical
-    pairs up to whole warps (484 cells, pml 6: two tiles of 121 pairs, 484 +
-    8 threads): one warp then carries both the physical and the absorbing
-    update.  Traces and images against the oracle."""
+    """Rows whose edges of gridphy lie inside a 32-column tile (484 cells,
+    pml 6): warps there hold gridphy's and absorbing cells.  Traces and
+    images against the oracle."""
     s = synth.small_case(n=(484, 10, 9), pml=6, nt=50, seed=17, shot_idx=[(240, 5, 3)])
     p = _problem(oracle, s)
     obs = oracle.forward(p)
@@ -437,8 +439,8 @@ def test_tile_with_a_mixed_warp(oracle, synth):
 
 @pytest.mark.parametrize("chunks", [1, 3, 7, 40])
 def test_run_chunks_change_no_result(synth, chunks):
-    """The run schedule of the persistent TMA kernels (run_chunks: chunks
-    of each tile's planes) only decides which CTA updates which cells, so
+    """The tile kernels' schedule (run_chunks: chunks of each tile's
+    planes) only decides which CTA updates which cells, so
     traces and images are bit-identical to the cost model's schedule; the
     chunking in use is reported (a count past the planes falls back to the
     cost model's)."""
