@@ -115,6 +115,15 @@ Status Engine::alloc(void **p, size_t bytes) {
     return Status{};
 }
 
+Status Engine::release(void *&p, size_t bytes) {
+    JV_CU(cudaFreeAsync(p, stream_));
+    JV_CU(cudaStreamSynchronize(stream_));
+    std::replace(allocs_.begin(), allocs_.end(), p, (void *)nullptr);
+    dev_bytes_ -= bytes;
+    p = nullptr;
+    return Status{};
+}
+
 Engine::~Engine() {
     if (stream_) {
         cudaSetDevice(dev_);
@@ -310,8 +319,9 @@ size_t footprint_bytes(const jv_grid &grid, int nt, int rec_width, bool rtm, int
     b += (kNumFld * fe + 32) * sizeof(float);                 // forward wavefield
     long long slabs = 0;
     make_pml_slabs(g, 1, &slabs);
-    const size_t psi = (size_t)(tiles_fit(g) ? tile_psi_floats(g) : slabs) * sizeof(float);
-    b += psi;                                                 // its memory variables
+    // its memory variables, in the layout of any kernel variant
+    const size_t psi = (size_t)std::max(tiles_fit(g) ? tile_psi_floats(g) : 0, slabs) * sizeof(float);
+    b += psi;
     b += 5 * nphy * sizeof(double);                           // stacks
     b += 16 * ((size_t)grid.nx + grid.ny + grid.nz + 2 * grid.pml * 3) + (1 << 20);  // tables, state, slack
     if (rtm) {
@@ -384,6 +394,10 @@ Status Engine::create(const jv_grid &grid, const float *vp, const float *vs, con
     // (autotune on, nothing fixed by hand) the result-neutral knobs only
     const bool neutral = !tune && opt.autotune && opt.run_chunks <= 0 && opt.tile_gx <= 0 && opt.tile_gy <= 0;
     if (s && (tune || neutral)) s = E->autotune(!tune);
+    // the measured choice has had both layouts of memory variables: keep the one in use
+    if (s && tune && E->tpsiF_)
+        s = E->tiles_ ? E->release((void *&)E->cpF_.psi, (size_t)E->psi_total_ * sizeof(float))
+                      : E->release((void *&)E->tpsiF_, (size_t)E->tpsi_total_ * sizeof(float));
     if (!s) {
         delete E;
         return s;

@@ -229,6 +229,7 @@ class Engine {
     std::map<long long, cudaGraphExec_t> graphs_;
 
     Status alloc(void **p, size_t bytes);
+    Status release(void *&p, size_t bytes);  // one of alloc's, and p
 
     // profiling state
     bool prof_ = false;

@@ -392,7 +392,9 @@ typedef struct jv_server_stats {
                                        requests kept the GPU                     */
 } jv_server_stats;
 /* Device bytes a context holds for one request of this size with n_recv
- * receivers and an FP32 boundary store (an estimate from the layout; the
+ * receivers and an FP32 boundary store (an estimate from the layout, for any
+ * kernel_variant; a measured choice, -1, holds the absorbing layers'
+ * memory variables twice while it is made; the
  * server's admission unit, which counts 2-byte records for a request with a
  * 16-bit store). */
 jv_status jv_footprint(const jv_grid *grid, int nt, int rec_width, int kind, int n_recv, size_t *bytes);

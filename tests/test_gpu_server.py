@@ -180,6 +180,19 @@ def test_footprint_covers_what_a_context_allocates():
         assert held <= est <= 1.3 * held + (4 << 20), (s.name, held, est)
 
 
+@pytest.mark.parametrize("variant", [-1, 0, 2, 3, 4])
+def test_footprint_covers_every_kernel_variant(variant):
+    """Variants 0 to 3 hold the slabs' memory variables, more than the tile kernels'; a context that has measured
+    its kernels holds one of the two; the receiver wavefield too."""
+    s = synth.small_case(n=(64, 56, 48), pml=16, nt=20, seed=15)
+    with jv.Context.from_survey(s, kernel_variant=variant) as ctx:
+        obs = ctx.forward(0)
+        ctx.rtm_shot(0, obs)
+        held = ctx.info().device_bytes
+    est = jv.footprint(s.nx, s.ny, s.nz, s.pml, s.nt, s.rec_width, jv.JOB_RTM, n_recv=len(s.recvs))
+    assert held <= est <= 1.3 * held, (variant, held, est)
+
+
 def test_cancel_and_timeout():
     big = synth.small_case(n=(48, 44, 40), pml=8, nt=1500, seed=14)
     small = _cases()[0]
