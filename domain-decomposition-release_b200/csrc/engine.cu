@@ -9,7 +9,6 @@
 #include "engine.hpp"
 
 #include <algorithm>
-#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -415,7 +414,7 @@ Status Engine::create(const jv_grid &grid, const float *vp, const float *vs, con
 // unless tile_gx / tile_gy were given, the float4 kernels' block shape: the default number of blocks per
 // gridphy row and one fewer or one more, timed on the reverse loop's
 // float4 velocity update and the backward stress update.  The fastest wins; the choice is
-// kept per grid shape and device for the contexts that follow.
+// kept per grid shape, device and options for the contexts that follow.
 Status Engine::autotune(bool neutral) {
     struct Cand {
         int variant, pml_minb, q;  // q: variant 4's run chunks
@@ -423,14 +422,15 @@ Status Engine::autotune(bool neutral) {
     };
     const bool shape_free = opt_.tile_gx <= 0 && opt_.tile_gy <= 0;
     static std::mutex mu;
-    static std::map<std::array<long long, 7>, Cand> cache;
+    static std::map<std::vector<long long>, Cand> cache;
     int dev = 0;
     JV_CU(cudaGetDevice(&dev));
     cudaDeviceProp prop{};
     JV_CU(cudaGetDeviceProperties(&prop, dev));
-    const std::array<long long, 7> key = {grid_.nx, grid_.ny, grid_.nz, grid_.pml, prop.multiProcessorCount,
-                                          (long long)prop.totalGlobalMem,
-                                          neutral ? 10 + kc_.variant : 0};
+    // the grid, the device, and the options that fix or limit a candidate
+    const std::vector<long long> key = {grid_.nx, grid_.ny, grid_.nz, grid_.pml, prop.multiProcessorCount,
+                                        (long long)prop.totalGlobalMem, neutral ? 10 + kc_.variant : 0,
+                                        opt_.run_chunks, opt_.tile_gx, opt_.tile_gy, kc_.minb, kc_.zp, kc_.pml_zp};
     Status st{};
     auto apply = [&](const Cand &c) {
         kc_.variant = c.variant;

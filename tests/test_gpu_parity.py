@@ -418,6 +418,18 @@ def test_measured_kernel_choice(oracle, synth):
         assert ctx.kernel_config()["kernel_variant"] == 4
 
 
+@pytest.mark.parametrize("first,second", [(0, 17), (17, 0)])
+def test_measured_choice_is_kept_per_options(synth, first, second):
+    """A chunking that one context fixes is not taken from, nor left to, a context of the same shape that does not
+    (17 chunks are none of the cost model's)."""
+    s = synth.small_case(n=(40, 24, 22 if first else 20), pml=9, nt=10, seed=63)
+    for q in (first, second):
+        with jv.Context.from_survey(s, kernel_variant=-1, run_chunks=q) as ctx:
+            cfg = ctx.kernel_config()
+        if cfg["kernel_variant"] == 4:
+            assert (cfg["run_chunks"] == 17) == (q == 17), (q, cfg["run_chunks"])
+
+
 def test_tile_with_a_mixed_warp(oracle, synth):
     """Rows whose edges of gridphy lie inside a 32-column tile (484 cells,
     pml 6): warps there hold gridphy's and absorbing cells.  Traces and
