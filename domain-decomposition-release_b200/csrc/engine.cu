@@ -568,7 +568,6 @@ Status Engine::alloc_all(const float *vp, const float *vs, const float *rho) {
         JV_TRY(alloc(&p, sizeof(int)));
         zm_err_ = (int *)p;
         JV_CU(cudaMemsetAsync(zm_err_, 0, sizeof(int), stream_));
-        JV_K(k_make_wave_maps(g_, F_, lam_, mu_, zm_err_, &mapsF_));
     }
 
     // CPML geometry: six slabs covering gridext outside gridphy and outside
@@ -591,9 +590,10 @@ Status Engine::alloc_all(const float *vp, const float *vs, const float *rho) {
         JV_TRY(make_tiles());
         tiles_ = tileF_.ok;
     }
-    // the slab layout's memory variables: the other variants, tried by the
-    // measured choice
+    // the slab layout's memory variables and variant 3's descriptors: the
+    // other variants, tried by the measured choice
     if (!tiles_ || opt_.kernel_variant < 0) {
+        if (kc_.variant >= 3) JV_K(k_make_wave_maps(g_, F_, lam_, mu_, zm_err_, &mapsF_));
         JV_TRY(alloc(&p, (size_t)psi_total_ * sizeof(float)));
         cpF_ = make_cpml((float *)p);
     }
@@ -1076,12 +1076,12 @@ Status Engine::rtm_prepare() {
         JV_TRY(alloc(&p, (kNumFld * field_elems_ + kGuard) * sizeof(float)));
         JV_CU(cudaMemsetAsync(p, 0, kGuard * sizeof(float), stream_));
         for (int f = 0; f < kNumFld; f++) R_.f[f] = (float *)p + kGuard + f * field_elems_;
-        if (kc_.variant >= 3) JV_K(k_make_wave_maps(g_, R_, lam_, mu_, zm_err_, &mapsR_));
         if (tiles_) {
             JV_TRY(alloc(&p, (size_t)tpsi_total_ * sizeof(float)));
             tpsiR_ = (float *)p;
             JV_TRY(make_tiles());
         } else {
+            if (kc_.variant >= 3) JV_K(k_make_wave_maps(g_, R_, lam_, mu_, zm_err_, &mapsR_));
             JV_TRY(alloc(&p, (size_t)psi_total_ * sizeof(float)));
             cpR_ = make_cpml((float *)p);
         }

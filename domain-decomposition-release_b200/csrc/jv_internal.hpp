@@ -177,10 +177,10 @@ int k_stress_phy(int mode, const GridDev &g, const WaveDev &w, const float *lam,
                  int rec_w, const float *wavelet, const StepState *st, int it_off, const KCfg &kc, void *stream,
                  const WaveMaps *maps = nullptr);
 // Builds the TMA descriptors of w's velocity fields for variant 3's
-// z-marching stress kernel (also variant 4's source reconstruction).  Rows
-// of more than 248 cells are cut into x tiles of an even number of pairs.
-// maps->ok stays false when those tiles would have fewer than 384 threads,
-// or the driver entry point is missing.  Returns a cudaError_t.
+// z-marching stress kernel.  Rows of more than 248 cells are cut into x tiles
+// of an even number of pairs.  maps->ok stays false when those tiles would
+// have fewer than 384 threads, or the driver entry point is missing.  Returns
+// a cudaError_t.
 int k_make_wave_maps(const GridDev &g, const WaveDev &w, const float *lam, const float *mu, int *err_flag,
                      WaveMaps *maps);
 int k_vel_pml(const GridDev &g, const CpmlDev &c, const WaveDev &w, const float *bdt, const float *vp,
