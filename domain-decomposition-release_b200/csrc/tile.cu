@@ -1038,26 +1038,38 @@ long long tile_psi_floats(const GridDev &g) {
     return 2 * 3 * (PX * ny * nz + PY * W * nz + PY * ny * W);
 }
 
-int k_make_tile_maps(const GridDev &g, const WaveDev &w, bool phy, float4 *const ax[3], float *psi, int *err_flag,
-                     int chunks, TileMaps *m) {
-    m->ok = false;
+TileGeo tile_geometry(const GridDev &g, bool phy) {
     TileGeo q{};
     const int n[3] = {g.nx, g.ny, g.nz}, p[3] = {g.px, g.py, g.pz};
     for (int a = 0; a < 3; a++) {
         q.lo[a] = phy ? g.m : 2;
         q.hi[a] = phy ? g.m + p[a] : n[a] - 2;
     }
-    int dev = 0, nsm = 0;
-    cudaGetDevice(&dev);
-    cudaError_t e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return (int)e;
-    if (!tiles_fit(g)) return 0;
     // tiles start on 128-byte lines: rows that straddle them measured 240
     // against 303 us (stress update, 200^3 + 20), more than the tile that a
     // shifted start can save
     q.e0 = ((int)g.xoff + q.lo[0]) / kTX * kTX;
     q.ntx = ((int)g.xoff + q.hi[0] - q.e0 + kTX - 1) / kTX;
     q.nty = (q.hi[1] - q.lo[1] + kTY - 1) / kTY;
+    const PsiCols c = psi_cols(g);
+    q.PX = round4(c.wl + c.wh);
+    q.PY = round4(c.wy);
+    q.W = 2 * (g.m - 2);
+    q.cxl = (int)g.xoff - c.xl;
+    q.cxh = c.wl + (int)g.xoff - c.xh;
+    q.cy = (int)g.xoff - c.yl;
+    return q;
+}
+
+int k_make_tile_maps(const GridDev &g, const WaveDev &w, bool phy, float4 *const ax[3], float *psi, int *err_flag,
+                     int chunks, TileMaps *m) {
+    m->ok = false;
+    TileGeo q = tile_geometry(g, phy);
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaError_t e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return (int)e;
+    if (!tiles_fit(g)) return 0;
     // planes per chunk: the work over two blocks an SM, a chunk's start
     // (barriers, the planes below and the first four above) costing about
     // five planes, and most of the last block's time, which the others wait
@@ -1088,13 +1100,6 @@ int k_make_tile_maps(const GridDev &g, const WaveDev &w, bool phy, float4 *const
     for (int k = 0; k < 3; k++) m->qcand[k] = qn[k];
     q.Q = chunks >= 1 && chunks <= nz ? chunks : qn[0];
     q.L = (nz + q.Q - 1) / q.Q;
-    const PsiCols c = psi_cols(g);
-    q.PX = round4(c.wl + c.wh);
-    q.PY = round4(c.wy);
-    q.W = 2 * (g.m - 2);
-    q.cxl = (int)g.xoff - c.xl;
-    q.cxh = c.wl + (int)g.xoff - c.xh;
-    q.cy = (int)g.xoff - c.yl;
     const long long nx3 = 3LL * q.PX * (g.ny - 4) * (g.nz - 4), ny3 = 3LL * q.PY * q.W * (g.nz - 4),
                     nz3 = 3LL * q.PY * (g.ny - 4) * q.W;
     for (int s = 0; s < 2; s++) {

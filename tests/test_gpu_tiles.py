@@ -6,6 +6,8 @@ thinnest layer, the source in a tile's corner cells.
 
 Tolerances are those of the other parity tests: traces 2e-5 and images 5e-5
 relative L2 (FP32 sums over some hundred time steps)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -184,39 +186,21 @@ def test_sums_of_differences_round_once(synth, n, dx, dy, dz):
         assert np.abs(img[k]).max() > 0 and np.array_equal(raw[k].astype(F32), img[k]), k
 
 
-def test_tile_layout_covers_every_cell():
-    """The columns of every grid fall in exactly one tile, start pairs on
-    8-byte boundaries, and the memory variables of a pair lie within their
-    row, for the offset make_layout picks (restated)."""
-    for m in range(4, 24):
-        for px in list(range(8, 76)) + [100, 160, 200, 338, 676]:
-            nx = px + 2 * m
-            tiles = lambda xo: (4 * ((xo + nx - 2 - (xo + 2) // 32 * 32 + 31) // 32)
-                                + 3 * ((xo + m + px - (xo + m) // 32 * 32 + 31) // 32))
-            x0 = (32 - m % 32) % 32
-            xoff = x0
-            for xo in range(x0 % 4, 32, 4):
-                if tiles(xo) < tiles(xoff):
-                    xoff = xo
-            assert (xoff + m) % 4 == 0
-            xl = (xoff + 2) & ~1
-            wl = ((xoff + m + 1) & ~1) - xl
-            xh = (xoff + m + px) & ~1
-            wh = ((xoff + nx - 1) & ~1) - xh
-            wy = ((xoff + nx - 1) & ~1) - xl
-            for lo, hi in ((2, nx - 2), (m, m + px)):
-                e0 = (xoff + lo) // 32 * 32
-                seen = set()
-                for e in range(e0, e0 + (xoff + hi - e0 + 31) // 32 * 32, 2):
-                    x = e - xoff
-                    cells = [c for c in (x, x + 1) if lo <= c < hi]
-                    assert not seen & set(cells)
-                    seen |= set(cells)
-                    if not cells or lo != 2:
-                        continue
-                    col = e - xl
-                    assert col % 2 == 0 and 0 <= col and col + 1 < wy
-                    if any(c < m or c >= m + px for c in cells):
-                        xc = e - xl if x < m else wl + e - xh
-                        assert xc % 2 == 0 and (0 <= xc < wl if x < m else wl <= xc < wl + wh)
-                assert seen == set(range(lo, hi))
+@pytest.mark.parametrize("n,pml", [((48, 20, 18), 10), ((32, 28, 24), 8), ((33, 9, 17), 5)])
+def test_tile_layout_covers_every_cell(synth, n, pml):
+    """jv_forward_noalloc runs the same kernels on rows as short as can be and the cost model's chunks: other row
+    offsets, tiles and chunks than a context's, and the same traces bit for bit, of receivers at every cell of two
+    planes (one along the layer's edge)."""
+    import torch
+    from test_zz_no_alloc import _run
+
+    s = synth.small_case(n=n, pml=pml, nt=60, seed=82)
+    s.recvs = (np.array([(i, j, k) for k in (0, n[2] // 2) for j in range(n[1]) for i in range(n[0])])
+               * np.array([s.dx, s.dy, s.dz])).astype(np.float32)
+    with jv.Context.from_survey(s, autotune=0, run_chunks=3) as ctx:
+        ref = ctx.forward(0)
+    out = torch.full((3, len(s.recvs), s.nt), float("nan"), dtype=torch.float32, device="cuda:0")
+    kept = ctypes.c_int(-1)
+    assert _run(s, out, kept) == jv.JV_OK and kept.value == len(s.recvs)
+    for a, b in zip(out.cpu().numpy(), ref):
+        assert np.abs(b).max() > 0 and np.array_equal(a, b)
