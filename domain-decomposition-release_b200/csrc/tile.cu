@@ -272,8 +272,9 @@ struct Place {
 // The planes of a block's march.  Event e delivers plane e + 4 of the fields
 // differenced in z (buffers A, four deeper than B) and plane e of the others
 // (buffers B) under one barrier; events -4 .. -1 only the former.  Plane k
-// is given back by one arrival of each live warp, and event e waits for
-// plane e - D: D planes are in flight or in use ahead of the four.
+// is given back by one arrival of each live warp, its lanes' reads fenced
+// against the copies that follow, and event e waits for plane e - D: D planes
+// are in flight or in use ahead of the four.
 template <int A_FLOATS, int B_FLOATS, int DEPTH>
 struct Flow {
     static constexpr int D = DEPTH, SA = DEPTH + 4;
@@ -323,6 +324,7 @@ struct Reader {
         return __all_sync(0xffffffffu, mbar_wait_bounded(flow.bars + 8u * s, (uint32_t)par));
     }
     __device__ __forceinline__ void release() const {
+        reads_before_bulk_copies();
         __syncwarp();
         if ((threadIdx.x & 31) == 0) mbar_arrive(flow.bars + 8u * (F::SA + b));
     }

@@ -34,6 +34,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
         if (clock64() - t0 > 2000000000LL) return false;
     }
 }
+// A thread's reads of shared memory come before the bulk copies that refill
+// it: executed by the reader before it gives the buffer back.  The barrier
+// alone orders only ordinary accesses; without the fence late reads met the
+// next plane (migrations of 144^3 differed from run to run in 31 of 200, with
+// two kernels on the chip in every one).
+__device__ __forceinline__ void reads_before_bulk_copies() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::

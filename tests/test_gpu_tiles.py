@@ -186,6 +186,25 @@ def test_sums_of_differences_round_once(synth, n, dx, dy, dz):
         assert np.abs(img[k]).max() > 0 and np.array_equal(raw[k].astype(F32), img[k]), k
 
 
+@pytest.mark.parametrize("precision", [jv.JV_FP32, jv.JV_FP16])
+def test_captured_migration_repeats_itself(synth, precision):
+    """A migration large enough to fill the chip, twelve times from captured graphs and three times from direct
+    launches: the same images, bit for bit.  A plane refilled under a late reader showed in every captured run."""
+    s = synth.scaled_cfg2(144, 160, pml=16)
+    out = []
+    for graphs in (1, 0):
+        with jv.Context.from_survey(s, use_graphs=graphs, precision=precision) as ctx:
+            tr = ctx.forward(0)
+            for _ in range(12 if graphs else 3):
+                ctx.image_reset()
+                ctx.rtm_shot(0, tr)
+                out.append((tr, ctx.images()))
+    for tr, im in out[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(tr, out[0][0]))
+        for k in im:
+            assert np.array_equal(im[k], out[0][1][k]), k
+
+
 @pytest.mark.parametrize("n,pml", [((48, 20, 18), 10), ((32, 28, 24), 8), ((33, 9, 17), 5)])
 def test_tile_layout_covers_every_cell(synth, n, pml):
     """jv_forward_noalloc runs the same kernels on rows as short as can be and the cost model's chunks: other row
