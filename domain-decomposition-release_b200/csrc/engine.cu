@@ -319,7 +319,7 @@ size_t footprint_bytes(const jv_grid &grid, int nt, int rec_width, bool rtm, int
     long long slabs = 0;
     make_pml_slabs(g, 1, &slabs);
     // its memory variables, in the layout of any kernel variant
-    const size_t psi = (size_t)std::max(tiles_fit(g) ? tile_psi_floats(g) : 0, slabs) * sizeof(float);
+    const size_t psi = (size_t)std::max(tile_psi_floats(g), slabs) * sizeof(float);
     b += psi;
     b += 5 * nphy * sizeof(double);                           // stacks
     b += 16 * ((size_t)grid.nx + grid.ny + grid.nz + 2 * grid.pml * 3) + (1 << 20);  // tables, state, slack
@@ -583,7 +583,7 @@ Status Engine::alloc_all(const float *vp, const float *vs, const float *rho) {
             JV_CU(cudaMemcpy(axis_d_[a], t[a].data(), t[a].size() * sizeof(float4), cudaMemcpyHostToDevice));
         }
     }
-    if (kc_.variant == 4 && tiles_fit(g_)) {
+    if (kc_.variant == 4) {
         tpsi_total_ = tile_psi_floats(g_);
         JV_TRY(alloc(&p, (size_t)tpsi_total_ * sizeof(float)));
         tpsiF_ = (float *)p;

@@ -40,8 +40,6 @@ struct TileMaps {
     int *err = nullptr;
 };
 
-// whether the tile kernels take a grid: they address arrays by 32-bit byte offsets
-inline bool tiles_fit(const GridDev &g) { return g.sz * g.nz < (1LL << 30); }
 // the region and tiles over gridext (phy false) or gridphy, and the places of
 // the memory variables: everything of a TileGeo that neither a device nor a
 // wavefield decides

@@ -84,8 +84,7 @@ typedef struct jv_options {
     int kernel_variant; /* stencil kernels: 0 one plane per block, 1 z-marching, 2 x-vectorised,
                            3 as 2 with a TMA-fed z-marching stress update, 4 (default) TMA-fed
                            z-marching tile kernels for every stencil update, the absorbing
-                           layers in the same kernels (grids whose arrays reach 4 GB run
-                           variant 3's kernels);
+                           layers in the same kernels;
                            -1: measured choice among 4, 3, 2, variant 4's run chunking,
                            the absorbing-layer register budget and the float4 kernels'
                            block shape on this grid at creation, kept per grid shape;

@@ -205,6 +205,30 @@ def test_captured_migration_repeats_itself(synth, precision):
             assert np.array_equal(im[k], out[0][1][k]), k
 
 
+def test_arrays_of_4_gb_and_more():
+    """A shot near the end of arrays of 4.4 GB, whose byte offsets pass 32 bits, against variant 3's kernels."""
+    import os
+    import torch
+
+    nx, ny, nz, pml, nt = 1000, 1000, 960, 20, 6
+    if torch.cuda.mem_get_info(0)[0] < 135e9 or os.sysconf("SC_AVPHYS_PAGES") * os.sysconf("SC_PAGE_SIZE") < 40e9:
+        pytest.skip("needs 125 GB of device memory and 30 GB of host memory")
+    vp = np.empty((nz, ny, nx), np.float32)
+    vp[:] = np.linspace(2000, 3000, nz, dtype=np.float32)[:, None, None]
+    vs, rho = vp / np.float32(1.732), np.full_like(vp, 2000)
+    shot = np.array([(nx // 2, ny // 2, nz - 6)])
+    recs = shot + np.array([(3 * i, 2 * j, -k) for i in (-2, 0, 2) for j in (0, 3) for k in (0, 5, 8)])
+    out = []
+    for variant in (4, 3):
+        with jv.Context.create(nx, ny, nz, pml, 5.0, 5.0, 5.0, vp, vs, rho, 4e-4, 100.0, nt, kernel_variant=variant,
+                               autotune=0) as ctx:
+            ctx.set_geometry((shot * 5.0).astype(np.float32), (recs * 5.0).astype(np.float32))
+            out.append(ctx.forward(0))
+            assert (ctx.kernel_config()["run_chunks"] > 0) == (variant == 4)
+    for a, b in zip(*out):
+        assert np.abs(b).max() > 0 and rel_l2(a, b) <= 1e-6  # sums of six steps in other orders
+
+
 @pytest.mark.parametrize("n,pml", [((48, 20, 18), 10), ((32, 28, 24), 8), ((33, 9, 17), 5)])
 def test_tile_layout_covers_every_cell(synth, n, pml):
     """jv_forward_noalloc runs the same kernels on rows as short as can be and the cost model's chunks: other row
