@@ -155,7 +155,11 @@ GridDev make_layout(const jv_grid &grid, size_t *field_elems, bool tight) {
     // lets the tile kernels' 32-column tiles, which start on such lines,
     // cover the rows with fewer tiles: four updates a migration step run over
     // gridext, three over gridphy.  Rows may grow by that where a field stays
-    // below 64 MB.
+    // below 64 MB: a migration step of n^3 + 10 then takes 281 against 299 us at
+    // n = 112, 465 against 498 at 144, 738 against 822 at 176 and 1158 against
+    // 1225 at 208, for 11 to 8 % more memory.  Above, it would still gain 4 %
+    // (1705 against 1777 at 240, 2395 against 2488 at 272), which is not worth
+    // 260 MB and more of a device that holds a boundary store.
     auto tiles = [&](int xo) {
         const int f = (xo + 2) / 32 * 32, p = (xo + m) / 32 * 32;
         return 4 * ((xo + g.nx - 2 - f + 31) / 32) + 3 * ((xo + m + g.px - p + 31) / 32);
@@ -411,10 +415,11 @@ Status Engine::create(const jv_grid &grid, const float *vp, const float *vs, con
 // fixes one), variant 3 where its stress kernel applies, variant 2 -- and,
 // for the variants with separate absorbing-layer kernels, their register
 // budget (3 or 4 blocks per SM).  Then, for a choice that runs them and
-// unless tile_gx / tile_gy were given, the float4 kernels' block shape: the default number of blocks per
-// gridphy row and one fewer or one more, timed on the reverse loop's
-// float4 velocity update and the backward stress update.  The fastest wins; the choice is
-// kept per grid shape, device and options for the contexts that follow.
+// unless tile_gx / tile_gy were given, the float4 kernels' block shape: the
+// default number of blocks per gridphy row and one fewer or one more, timed
+// on the reverse loop's float4 velocity update and the backward stress
+// update.  The fastest wins; the choice is kept per grid shape, device and
+// options for the contexts that follow.
 Status Engine::autotune(bool neutral) {
     struct Cand {
         int variant, pml_minb, q;  // q: variant 4's run chunks
@@ -1341,7 +1346,7 @@ Status Engine::check_zm_err() {
     JV_CU(cudaMemcpy(&h, zm_err_, sizeof(int), cudaMemcpyDeviceToHost));
     if (h) {
         JV_CU(cudaMemset(zm_err_, 0, sizeof(int)));
-        return bad(JV_ETIMEOUT, "a shared-memory tile of the z-marching stress kernel did not arrive in time");
+        return bad(JV_ETIMEOUT, "a shared-memory tile of a TMA-fed kernel did not arrive in time");
     }
     return Status{};
 }

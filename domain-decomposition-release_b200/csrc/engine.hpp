@@ -188,7 +188,7 @@ class Engine {
 
   private:
     bool tiles_ = false;          // the time loops run variant 4's tile kernels
-    int *zm_err_ = nullptr;       // device flag of variant 3's bounded waits
+    int *zm_err_ = nullptr;       // device flag of the TMA-fed kernels' bounded waits (variants 3 and 4)
     Status check_zm_err();
     size_t field_elems_ = 0;  // elements per pitched field
     std::vector<void *> allocs_;

@@ -8,8 +8,9 @@
 //   so that the first gridphy column (i = pml) starts on a 16-byte boundary,
 //   on a 128-byte one unless the tile kernels cover the rows with fewer
 //   tiles otherwise.
-//   Absorbing-layer memory variables live only in the six boundary slabs
-//   (slab-local dense indexing), not on the full grid.
+//   Absorbing-layer memory variables are kept for the cells that absorb only:
+//   per axis for the tile kernels (tile.hpp), in the six boundary slabs
+//   (slab-local dense indexing) for the other variants.
 #pragma once
 
 #include <cstddef>

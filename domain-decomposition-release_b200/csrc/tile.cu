@@ -15,19 +15,30 @@
 //   imaging             RTM/rtm3d_0_image_module/rtm3d_iamge_kernel.hpp:6-51
 //
 // Shape.  Eight warps own a tile of 32 x 16 cells, one x pair per thread, and
-// march it through a chunk of z planes.  x and y neighbours come from shared memory, where TMA brings each plane of the
-// differenced fields with its 4-cell halo.  A field that is also differenced
-// in z arrives four planes ahead, so that the planes above are read from
-// the same buffers and only the three or four planes below are carried in
-// registers.  What a cell reads alone (model, the updated fields) goes
-// straight to registers, behind an L2 prefetch a plane ahead.  A warp
-// gives a plane back with one arrival once its differences are taken and
-// runs on; nothing in the loop waits for the slowest warp of the block, and
-// two blocks share an SM.
+// march it through a chunk of z planes.  x and y neighbours come from shared
+// memory, where TMA brings each plane of the differenced fields with its
+// 4-cell halo.  A field that is also differenced in z arrives four planes
+// ahead, so that the planes above are read from the same buffers and only the
+// three or four planes below are carried in registers.  What a cell reads
+// alone (model, the updated fields) goes straight to registers, behind an L2
+// prefetch a plane ahead.  A warp gives a plane back with one arrival once its
+// differences are taken and runs on; nothing in the loop waits for the slowest
+// warp of the block, and two blocks share an SM.
 //
 // Cells of the absorbing layers take the same 8-tap differences with their
 // outer two weights zero, so a warp that holds both kinds does not run two
-// paths; only the memory variables are a branch.
+// paths; the memory variables and the rounding of the sums are branches.
+//
+// What bounds them, 200^3 + 20 (us, and GB/s of arrays read and written once;
+// a copy moves 6460): with absorbing layers instruction issue, 0.5 a cycle and
+// scheduler -- stress 272 (4280), velocity 237 (3590), against 259 and 227 for
+// the persistent kernels of one CTA an SM that they replaced, with a separate
+// launch for wide or odd grids; over gridphy DRAM latency -- imaging with
+// P-wave velocities 192 (5160), backward stress 133 (4590), backward velocity
+// 113 (3690), against 250 for imaging with the backward velocity update, 147
+// for the backward stress and 147 + 124 for the receivers' velocity update and
+// its layers.  The 200^3 migration gains 3 %, small, odd and wide grids 10 to
+// 100 %.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
@@ -1071,12 +1082,14 @@ int k_make_tile_maps(const GridDev &g, const WaveDev &w, bool phy, float4 *const
     cudaGetDevice(&dev);
     cudaError_t e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return (int)e;
-    // planes per chunk: the work over two blocks an SM, a chunk's start
-    // (barriers, the planes below and the first four above) costing about
-    // five planes, and most of the last block's time, which the others wait
-    // for (a block in a corner of the absorbing layers takes twice as long as
-    // one of gridphy, so that a single wave of long chunks is the worst split:
-    // 160^3 + 16, 4 chunks against 10, 986 against 830 us a migration step)
+    // Planes per chunk.  Over gridphy: waves of two blocks an SM, a chunk's
+    // start (barriers, the planes below and the first four above) costing
+    // about ten of its planes.  Over gridext a plane costs more, the start
+    // about five, and blocks differ: one in a corner of the absorbing layers
+    // takes twice as long as one of gridphy, so that the others wait for most
+    // of the last block (0.8 of one) and a single wave of long chunks is the
+    // worst split (160^3 + 16, 4 chunks against 10, 986 against 830 us a
+    // migration step).
     const int nz = q.hi[2] - q.lo[2];
     const long long slots = 2 * nsm;
     long long qc[3] = {-1, -1, -1};
